@@ -4,6 +4,42 @@
 
 namespace {
 
+// Division of a 32-bit index by a run-time constant as a multiply-high and a shift (Granlund & Montgomery, "Division by
+// invariant integers using multiplication", 1994): exact for every numerator below 2^31.
+struct FastDiv {
+  unsigned d, mul, shift;
+  explicit FastDiv(unsigned v = 1) : d(v) {
+    shift = 0; while ((1ull << shift) < v) ++shift;
+    mul = (unsigned)(((1ull << 32) * ((1ull << shift) - v)) / v + 1);
+  }
+  __device__ __forceinline__ unsigned div(unsigned n) const { return (__umulhi(n, mul) + n) >> shift; }
+};
+
+// Axis swap that leaves the innermost `inner` elements together: y[o][j][m][i][:] = x[o][i][m][j][:] -- the attention
+// layout change [B,S,H,d] -> [B,H,S,d] and back.  V is the widest vector that divides a run; every thread moves four
+// vectors, all loads before the first store.  Bound by HBM: [1024,64,8,32] (67 MB each way) 109 -> 23 us, where one
+// element per thread and six 64-bit divisions each was bound by the arithmetic.
+struct SwapArgs { FastDiv run, dlo, mid, dhi; unsigned s_o, s_i, s_m, s_j; };     // vectors per run, extents, input strides in vectors
+template <typename V>
+__global__ void __launch_bounds__(256)
+swap_axes_kernel(const V* __restrict__ x, V* __restrict__ y, unsigned n, SwapArgs a) {
+  V v[4];
+  const unsigned first = blockIdx.x * 1024 + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const unsigned idx = first + k * 256;
+    if (idx < n) {
+      unsigned q = a.run.div(idx), src = idx - q * a.run.d, t = a.dlo.div(q);      // output order: [outer][dhi][mid][dlo][run]
+      src += (q - t * a.dlo.d) * a.s_i; q = a.mid.div(t);
+      src += (t - q * a.mid.d) * a.s_m; t = a.dhi.div(q);
+      src += (q - t * a.dhi.d) * a.s_j + t * a.s_o;
+      v[k] = x[src];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) { const unsigned idx = first + k * 256; if (idx < n) y[idx] = v[k]; }
+}
+
 struct TransposeArgs { long long in_stride[6]; long long out_shape[6]; int rank; };
 
 // General axis swap.  Each thread produces one output element; when the innermost axis is
@@ -48,6 +84,37 @@ __global__ void split_last_kernel(const float* __restrict__ g, float* __restrict
   long long r = idx / w; int c = (int)(idx % w); float v = g[idx];
   if (c < da) { if (ga) { long long o = r * da + c; ga[o] = acc ? ga[o] + v : v; } }
   else if (gb) { long long o = r * db + (c - da); gb[o] = acc ? gb[o] + v : v; }
+}
+// Vector forms (both widths a multiple of four, 16-byte aligned): a thread moves four float4, loads before stores.  Bound by
+// HBM: splitting [65536, 768] into 256 | 512 160 -> 62 us.
+__global__ void __launch_bounds__(256)
+concat_last_vec_kernel(const float4* __restrict__ a, const float4* __restrict__ b, float4* __restrict__ out, unsigned n, FastDiv width, unsigned da) {
+  const unsigned first = blockIdx.x * 1024 + threadIdx.x, db = width.d - da;
+  float4 v[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const unsigned idx = first + k * 256;
+    if (idx < n) { const unsigned r = width.div(idx), c = idx - r * width.d; v[k] = c < da ? a[r * da + c] : b[r * db + (c - da)]; }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) { const unsigned idx = first + k * 256; if (idx < n) out[idx] = v[k]; }
+}
+__global__ void __launch_bounds__(256)
+split_last_vec_kernel(const float4* __restrict__ g, float4* __restrict__ ga, float4* __restrict__ gb, unsigned n, FastDiv width, unsigned da, int acc) {
+  const unsigned first = blockIdx.x * 1024 + threadIdx.x, db = width.d - da;
+  float4 v[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) { const unsigned idx = first + k * 256; if (idx < n) v[k] = g[idx]; }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const unsigned idx = first + k * 256;
+    if (idx >= n) continue;
+    const unsigned r = width.div(idx), c = idx - r * width.d;
+    float4* dst = c < da ? (ga ? ga + (r * da + c) : nullptr) : (gb ? gb + (r * db + (c - da)) : nullptr);
+    if (!dst) continue;
+    if (acc) { const float4 o = *dst; v[k].x += o.x; v[k].y += o.y; v[k].z += o.z; v[k].w += o.w; }
+    *dst = v[k];
+  }
 }
 __global__ void last_token_kernel(const float* __restrict__ x, float* __restrict__ y, long long B, long long S, int D) {
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -103,11 +170,32 @@ __global__ void ew_unary_bwd_kernel(int op, const float* __restrict__ x, const f
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dx[i] += dy[i] * ew_bwd(op, x[i], p0, p1);
 }
-__global__ void ew_binary_kernel(int op, const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ y, long long n) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float u = a[i], v = b[i];
-  y[i] = op == TALOS_EW_ADD ? u + v : op == TALOS_EW_SUB ? u - v : op == TALOS_EW_MUL ? u * v : u / v;
+__device__ __forceinline__ float ew_binary(int op, float u, float v) {
+  return op == TALOS_EW_ADD ? u + v : op == TALOS_EW_SUB ? u - v : op == TALOS_EW_MUL ? u * v : u / v;
+}
+// V: float4 when the three buffers are 16-byte aligned (n is then the count of whole vectors and one extra block does the
+// last n % 4 elements), float otherwise.  Two vectors a thread: the residual add of [65536, 256] runs at the copy rate
+// (57 -> 30 us; one float a thread was bound by instructions and by too few bytes in flight).
+template <typename V>
+__global__ void __launch_bounds__(256)
+ew_binary_kernel(int op, const V* a, const V* b, V* y, long long n, int rest) {
+  if (rest && blockIdx.x == gridDim.x - 1) {
+    const float *at = (const float*)(a + n), *bt = (const float*)(b + n); float* yt = (float*)(y + n);
+    if ((int)threadIdx.x < rest) yt[threadIdx.x] = ew_binary(op, at[threadIdx.x], bt[threadIdx.x]);
+    return;
+  }
+  const long long i = (long long)blockIdx.x * 512 + threadIdx.x;
+  V u[2], v[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) if (i + k * 256 < n) { u[k] = a[i + k * 256]; v[k] = b[i + k * 256]; }
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    if (i + k * 256 < n) {
+      V o; const float *uf = (const float*)&u[k], *vf = (const float*)&v[k];
+#pragma unroll
+      for (int c = 0; c < (int)(sizeof(V) / 4); ++c) ((float*)&o)[c] = ew_binary(op, uf[c], vf[c]);
+      y[i + k * 256] = o;
+    }
 }
 // da/db may alias (x op x): both contributions are then added by the same thread in turn.
 __global__ void ew_binary_bwd_kernel(int op, const float* a, const float* b, const float* __restrict__ dy, float* da, float* db, long long n) {
@@ -147,6 +235,7 @@ __global__ void fill_from_scalar_kernel(const float* __restrict__ s, float scale
 }
 
 inline unsigned blocks_for(int64_t n) { return (unsigned)ceil_div(n, 256); }
+inline bool aligned_to(size_t bytes, const void* a, const void* b, const void* c = nullptr) { return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & (bytes - 1)) == 0; }
 
 }  // namespace
 
@@ -168,6 +257,21 @@ TALOS_API talos_status talos_transpose(talos_ctx* ctx, const float* x, float* y,
       return TALOS_OK;
     }
   }
+  if (lo != hi && hi < rank - 1 && !accumulate && n < (1LL << 31)) {
+    int64_t inner = 1, mid = 1, outer_n = 1;
+    for (int i = hi + 1; i < rank; ++i) inner *= shape[i];
+    for (int i = lo + 1; i < hi; ++i) mid *= shape[i];
+    for (int i = 0; i < lo; ++i) outer_n *= shape[i];
+    const int vec = (inner % 4 == 0 && aligned_to(16, x, y)) ? 4 : (inner % 2 == 0 && aligned_to(8, x, y)) ? 2 : 1;
+    const unsigned run = (unsigned)(inner / vec), total = (unsigned)(n / vec), grid = (unsigned)ceil_div(total, 1024);
+    const unsigned sj = run, sm = sj * (unsigned)shape[hi], si = sm * (unsigned)mid, so = si * (unsigned)shape[lo];
+    const SwapArgs g{FastDiv(run), FastDiv((unsigned)shape[lo]), FastDiv((unsigned)mid), FastDiv((unsigned)shape[hi]), so, si, sm, sj};
+    if (vec == 4) swap_axes_kernel<float4><<<grid, 256, 0, ctx->stream>>>((const float4*)x, (float4*)y, total, g);
+    else if (vec == 2) swap_axes_kernel<float2><<<grid, 256, 0, ctx->stream>>>((const float2*)x, (float2*)y, total, g);
+    else swap_axes_kernel<float><<<grid, 256, 0, ctx->stream>>>(x, y, total, g);
+    talos_launched(ctx, "transpose");
+    return TALOS_OK;
+  }
   TransposeArgs a; a.rank = rank;
   long long in_stride[6], st = 1;
   for (int i = rank - 1; i >= 0; --i) { in_stride[i] = st; st *= shape[i]; }
@@ -185,6 +289,12 @@ TALOS_API talos_status talos_concat_last(talos_ctx* ctx, const float* a, const f
   TALOS_REQUIRE(rows >= 0 && da >= 0 && db >= 0 && da + db < (1 << 30), TALOS_ERR_SHAPE, "bad concat shape");
   int64_t n = rows * (da + db); if (n == 0) return TALOS_OK;
   TALOS_REQUIRE(a && b && out, TALOS_ERR_ARG, "null pointer");
+  if (da % 4 == 0 && db % 4 == 0 && n < (1LL << 31) && aligned_to(16, a, b, out)) {
+    concat_last_vec_kernel<<<(unsigned)ceil_div(n / 4, 1024), 256, 0, ctx->stream>>>((const float4*)a, (const float4*)b, (float4*)out, (unsigned)(n / 4),
+                                                                                    FastDiv((unsigned)((da + db) / 4)), (unsigned)(da / 4));
+    talos_launched(ctx, "concat_last");
+    return TALOS_OK;
+  }
   concat_last_kernel<<<blocks_for(n), 256, 0, ctx->stream>>>(a, b, out, rows, (int)da, (int)db);
   talos_launched(ctx, "concat_last");
   TALOS_ENTRY_END
@@ -195,6 +305,12 @@ TALOS_API talos_status talos_split_last(talos_ctx* ctx, const float* g, float* g
   TALOS_REQUIRE(rows >= 0 && da >= 0 && db >= 0 && da + db < (1 << 30), TALOS_ERR_SHAPE, "bad split shape");
   int64_t n = rows * (da + db); if (n == 0) return TALOS_OK;
   TALOS_REQUIRE(g, TALOS_ERR_ARG, "null pointer");
+  if (da % 4 == 0 && db % 4 == 0 && n < (1LL << 31) && aligned_to(16, g, ga, gb)) {
+    split_last_vec_kernel<<<(unsigned)ceil_div(n / 4, 1024), 256, 0, ctx->stream>>>((const float4*)g, (float4*)ga, (float4*)gb, (unsigned)(n / 4),
+                                                                                   FastDiv((unsigned)((da + db) / 4)), (unsigned)(da / 4), accumulate ? 1 : 0);
+    talos_launched(ctx, "split_last");
+    return TALOS_OK;
+  }
   split_last_kernel<<<blocks_for(n), 256, 0, ctx->stream>>>(g, ga, gb, rows, (int)da, (int)db, accumulate ? 1 : 0);
   talos_launched(ctx, "split_last");
   TALOS_ENTRY_END
@@ -246,7 +362,12 @@ TALOS_API talos_status talos_eltwise_binary(talos_ctx* ctx, int32_t op, const fl
   TALOS_REQUIRE(op >= TALOS_EW_ADD && op <= TALOS_EW_DIV, TALOS_ERR_ARG, "bad binary op");
   TALOS_REQUIRE(n >= 0, TALOS_ERR_SHAPE, "negative length"); if (n == 0) return TALOS_OK;
   TALOS_REQUIRE(a && b && y, TALOS_ERR_ARG, "null pointer");
-  ew_binary_kernel<<<blocks_for(n), 256, 0, ctx->stream>>>(op, a, b, y, n);
+  if (aligned_to(16, a, b, y)) {
+    const int64_t n4 = n / 4; const int rest = (int)(n & 3);
+    ew_binary_kernel<float4><<<(unsigned)(ceil_div(n4, 512) + (rest ? 1 : 0)), 256, 0, ctx->stream>>>(op, (const float4*)a, (const float4*)b, (float4*)y, n4, rest);
+  } else {
+    ew_binary_kernel<float><<<(unsigned)ceil_div(n, 512), 256, 0, ctx->stream>>>(op, a, b, y, n, 0);
+  }
   talos_launched(ctx, "eltwise_binary");
   TALOS_ENTRY_END
 }

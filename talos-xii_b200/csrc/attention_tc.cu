@@ -242,7 +242,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 // 16-byte aligned operands; the four tiles must fit in shared memory.
 bool talos_attention_tc_fused(talos_ctx* ctx, const float* q, const float* k, const float* v, float* out, float* probs, int64_t BH,
                               int64_t S, int64_t dqk, int64_t dv, float scale, int causal) {
-  if (getenv("TALOS_ATTN_NO_FUSED")) return false;
+  if (talos_switches() & SW_ATTN_NO_FUSED) return false;
   if (S < 32 || S > 128 || (S & 31) || (dqk & 31) || (dv & 31) || dqk < 32 || dqk > 128 || dv < 32 || dv > S || BH < 1 || BH >= (1 << 30)) return false;
   if ((((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out | (uintptr_t)probs) & 15) != 0) return false;
   const size_t smem = (size_t)(dqk / 32) * (BM * 128 + S * 128) + (size_t)(S / 32) * ((dv / 32) * 4096 + BM * 128) + 16 * 8 + 1024;
@@ -259,7 +259,8 @@ bool talos_attention_tc_fused(talos_ctx* ctx, const float* q, const float* k, co
   AttnArgs g;
   g.BH = (int)BH; g.S = (int)S; g.dqk = (int)dqk; g.dv = (int)dv; g.scale_log2e = scale * 1.4426950408889634f; g.causal = causal; g.want_probs = probs ? 1 : 0;
   g.status = ctx->dev_status; g.wait_spins = ctx->dbg_wait_spins ? ctx->dbg_wait_spins : WAIT_SPINS;
-  TALOS_CHECK_CUDA(cudaFuncSetAttribute(attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static std::atomic<uint64_t> smem_set{0};
+  talos_allow_smem(smem_set, (const void*)attention_tc_kernel, 227 * 1024, ctx->device);
   const int grid = (int)std::min<int64_t>(BH, ctx->sm_count);
   attention_tc_kernel<<<grid, ATT_THREADS, smem, ctx->stream>>>(tq, tk, tv, to, tp, g);
   talos_launched(ctx, "attention_tc_fused");

@@ -92,6 +92,22 @@ inline void talos_launched(talos_ctx* ctx, const char* what) {
   if (ctx->timeline) talos_timeline_mark(ctx, what);
 }
 
+// The measurement switches (environment variables TALOS_*) that are set right now, as a bit mask: ONE walk over the
+// environment per call instead of one per switch (a dozen getenv calls were 1.5 us of every tensor-core launch).
+enum : unsigned {
+  SW_DISABLE_TENSOR_CORES = 1u << 0, SW_TC_NO_SHORTK = 1u << 1, SW_TC_NO_WIDE_EPI = 1u << 2, SW_TC_NO_EARLY = 1u << 3, SW_TC_NO_PREFETCH = 1u << 4,
+  SW_TC_FORCE_PAIR = 1u << 5, SW_TC_NO_PAIR = 1u << 6, SW_TC_NO_RASTER = 1u << 7, SW_TC_NO_FOLD = 1u << 8, SW_TC_NO_FUSED_DACT = 1u << 9,
+  SW_TC_NO_EPI8 = 1u << 10, SW_ATTN_NO_FUSED = 1u << 11, SW_TC_NO_SMALL = 1u << 12
+};
+unsigned talos_switches();
+// Raises a kernel's dynamic shared memory limit once per device (`done`: one bit per device, a static of the launcher).
+inline void talos_allow_smem(std::atomic<uint64_t>& done, const void* kern, size_t bytes, int device) {
+  const uint64_t bit = 1ull << (device & 63);
+  if (device < 64 && (done.load(std::memory_order_acquire) & bit)) return;
+  TALOS_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  done.fetch_or(bit, std::memory_order_release);
+}
+
 static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // ---- activation helpers shared by the GEMM epilogues and the elementwise kernels ----
@@ -148,6 +164,10 @@ __device__ __forceinline__ float talos_epilogue_apply(const EpiArgs& e, float ac
 void talos_gemm_fp32_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K, const float* A,
                             int64_t lda, int64_t strideA, const float* B, int64_t ldb, int64_t strideB, float* C,
                             int64_t ldc, int64_t strideC, int64_t batch, const EpiArgs& epi);
+void talos_gemm_small_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, int64_t strideA, const float* B,
+                             int64_t ldb, int64_t strideB, float* C, int64_t ldc, int64_t strideC, int64_t batch, const EpiArgs& epi);
+void talos_linear_bwd_small_launch(talos_ctx* ctx, const float* x, const float* W, const float* saved, const float* dy, float* dx, float* dW, float* db,
+                                   int64_t rows, int64_t in_f, int64_t out_f, int act, int accumulate);
 // Returns false when the shape/alignment is not eligible (caller falls back to the fp32 kernel).
 // First stage of the column sums only: dZ = dY * act'(saved) when dact != 0 (dz may alias dy) and the per-slab column
 // sums of dZ left in `partial` ([slabs][n]); returns the slab count, 0 (nothing launched) when the shape is not served.

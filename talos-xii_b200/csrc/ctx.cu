@@ -14,6 +14,21 @@ void talos_set_last_error(const std::string& msg) { g_last_error = msg; }
 
 TALOS_API const char* talos_last_error_string(void) { return g_last_error.c_str(); }
 
+extern char** environ;
+unsigned talos_switches() {
+  static const struct { const char* name; unsigned bit; } names[] = {
+      {"DISABLE_TENSOR_CORES", SW_DISABLE_TENSOR_CORES}, {"TC_NO_SHORTK", SW_TC_NO_SHORTK}, {"TC_NO_WIDE_EPI", SW_TC_NO_WIDE_EPI}, {"TC_NO_EARLY", SW_TC_NO_EARLY},
+      {"TC_NO_PREFETCH", SW_TC_NO_PREFETCH}, {"TC_FORCE_PAIR", SW_TC_FORCE_PAIR}, {"TC_NO_PAIR", SW_TC_NO_PAIR}, {"TC_NO_RASTER", SW_TC_NO_RASTER},
+      {"TC_NO_FOLD", SW_TC_NO_FOLD}, {"TC_NO_FUSED_DACT", SW_TC_NO_FUSED_DACT}, {"TC_NO_EPI8", SW_TC_NO_EPI8}, {"ATTN_NO_FUSED", SW_ATTN_NO_FUSED}, {"TC_NO_SMALL", SW_TC_NO_SMALL}};
+  unsigned mask = 0;
+  for (char** e = environ; e && *e; ++e) {
+    const char* v = *e;
+    if (v[0] != 'T' || strncmp(v, "TALOS_", 6) != 0) continue;
+    for (const auto& n : names) { const size_t l = strlen(n.name); if (strncmp(v + 6, n.name, l) == 0 && v[6 + l] == '=') mask |= n.bit; }
+  }
+  return mask;
+}
+
 static void* grow_scratch(talos_ctx* ctx, void** buf, size_t* have, size_t bytes) {
   if (bytes <= *have) return *buf;
   size_t want = bytes + (bytes >> 2);

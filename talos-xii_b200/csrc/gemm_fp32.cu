@@ -182,32 +182,33 @@ void talos_splitk_reduce(talos_ctx* ctx, const float* partial, int splits, int64
 void talos_gemm_fp32_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K, const float* A,
                             int64_t lda, int64_t strideA, const float* B, int64_t ldb, int64_t strideB, float* C,
                             int64_t ldc, int64_t strideC, int64_t batch, const EpiArgs& epi) {
+  // The 128 x 128 kernel takes products that give at least half of the SMs a tile, or whose long reduction it can split to do
+  // so (the weight-gradient shape: M, N <= 256 with K = the minibatch); everything smaller goes to the small kernel, and so
+  // do short reductions, where this one is all scattered epilogue (8 192 x 256 x 16: 28 against 8 us).
+  const int64_t tiles = ceil_div(M, 128) * ceil_div(N, 128) * batch;
+  int splits = 1;
+  if (batch == 1 && tiles * 2 <= ctx->sm_count && K >= 2048) {
+    splits = (int)std::min<int64_t>(ceil_div(2 * ctx->sm_count, tiles), K / 512);
+    if (splits < 2) splits = 1;
+  }
+  if (!(M >= 96 && N >= 96) || K < 256 || (tiles * 2 < ctx->sm_count && splits == 1)) {
+    talos_gemm_small_launch(ctx, opA, opB, M, N, K, A, lda, strideA, B, ldb, strideB, C, ldc, strideC, batch, epi);
+    return;
+  }
   GemmArgs g;
   g.A = A; g.B = B; g.C = C; g.ldc = ldc;
   g.sAm = opA == TALOS_OP_N ? lda : 1; g.sAk = opA == TALOS_OP_N ? 1 : lda;
   g.sBk = opB == TALOS_OP_N ? ldb : 1; g.sBn = opB == TALOS_OP_N ? 1 : ldb;
   g.batchA = strideA; g.batchB = strideB; g.batchC = strideC;
   g.M = (int)M; g.N = (int)N; g.K = (int)K; g.k_chunk = (int)K; g.splits = 1; g.partial = nullptr; g.epi = epi;
-
-  const bool big = (M >= 96 && N >= 96);
-  const int BM = big ? 128 : 64, BN = big ? 128 : 64;
-  int64_t tiles = ceil_div(M, BM) * ceil_div(N, BN) * batch;
-  // Split the reduction when the output has too few tiles to fill the machine (the dW shape:
-  // M,N <= 256 with K = the minibatch).
-  int splits = 1;
-  if (batch == 1 && tiles * 2 <= ctx->sm_count && K >= 2048) {
-    splits = (int)std::min<int64_t>(ceil_div(2 * ctx->sm_count, tiles), K / 512);
-    if (splits < 2) splits = 1;
-  }
   if (splits > 1) {
     int chunk = (int)ceil_div(K, splits); chunk = (chunk + 15) / 16 * 16;
     splits = (int)ceil_div(K, chunk);
     g.k_chunk = chunk; g.splits = splits;
     g.partial = (float*)talos_workspace(ctx, sizeof(float) * (size_t)splits * M * N);
   }
-  dim3 grid((unsigned)ceil_div(N, BN), (unsigned)ceil_div(M, BM), (unsigned)(splits > 1 ? splits : batch));
-  if (big) gemm_fp32_kernel<128, 128, 16, 8, 8><<<grid, 256, 0, ctx->stream>>>(g);
-  else gemm_fp32_kernel<64, 64, 16, 4, 4><<<grid, 256, 0, ctx->stream>>>(g);
+  dim3 grid((unsigned)ceil_div(N, 128), (unsigned)ceil_div(M, 128), (unsigned)(splits > 1 ? splits : batch));
+  gemm_fp32_kernel<128, 128, 16, 8, 8><<<grid, 256, 0, ctx->stream>>>(g);
   talos_launched(ctx, "gemm_fp32");
   if (splits > 1) talos_splitk_reduce(ctx, g.partial, splits, M, N, C, ldc, epi);
 }

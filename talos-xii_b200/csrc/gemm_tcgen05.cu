@@ -470,7 +470,8 @@ template <int BN, int STAGES, bool X3, bool A_MN, bool B_MN, int MINB = 1, bool 
 void launch_one(talos_ctx* ctx, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tbl, const TcArgs& g, int grid) {
   auto kern = gemm_tc_kernel<BN, STAGES, X3, A_MN, B_MN, MINB, BPS, SBUF, EW>;
   size_t smem = tc_smem_bytes<BN, STAGES, X3, SBUF, EW>();
-  TALOS_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static std::atomic<uint64_t> smem_set{0};
+  talos_allow_smem(smem_set, (const void*)kern, smem, ctx->device);
   kern<<<grid, TcRoles<X3, BPS, BN, EW>::THREADS, smem, ctx->stream>>>(ta, tb, tc, tbl, g);
   talos_launched(ctx, "gemm_tcgen05");
 }
@@ -495,27 +496,28 @@ void tc_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K
                int64_t ldb, float* C, int64_t ldc, int mode, const EpiArgs& epi, const TcBatch& bt = TcBatch{1, 0, 0, 0},
                const TcExtra* extra = nullptr) {
   const bool batched = bt.batch > 1;
+  const unsigned sw = talos_switches();
   const bool b_given = extra && extra->b_hi && !batched && (x3_mode(mode) ? extra->b_lo != nullptr : true);
   const bool a_mn = (opA == TALOS_OP_T), b_mn = (opB == TALOS_OP_N), x3 = (mode == TALOS_MODE_TF32X3);
   int bn = N > 128 ? 256 : N > 64 ? 128 : N > 32 ? 64 : 32;
   // Short reductions with a prepared small B (K <= 64: the first layer's forward product) are all epilogue: 128-column
   // tiles leave the shared memory for two staging buffers per epilogue warp, so that the store engine's read of one
   // chunk overlaps the arithmetic of the next.
-  const bool short_k = !batched && x3 && bn == 256 && K <= 64 && (b_given || (opB == TALOS_OP_N ? K * N : N * K) <= (1 << 20)) && !getenv("TALOS_TC_NO_SHORTK");
+  const bool short_k = !batched && x3 && bn == 256 && K <= 64 && (b_given || (opB == TALOS_OP_N ? K * N : N * K) <= (1 << 20)) && !(sw & SW_TC_NO_SHORTK);
   if (short_k) bn = 128;
   // (that configuration is all epilogue: sixteen epilogue warps, one 32-column chunk of a tile each, instead of eight with two)
-  const bool wide_epi = short_k && !getenv("TALOS_TC_NO_WIDE_EPI");
+  const bool wide_epi = short_k && !(sw & SW_TC_NO_WIDE_EPI);
   TcArgs g;
   g.M = (int)M; g.N = (int)N; g.K = (int)K; g.C = C; g.ldc = ldc; g.epi = epi; g.status = ctx->dev_status; g.partial = nullptr;
   g.batch = (int)std::max<int64_t>(bt.batch, 1); g.stride_c = batched ? bt.stride_c : 0;
-  g.early_pass = getenv("TALOS_TC_NO_EARLY") ? 0 : 1;
+  g.early_pass = (sw & SW_TC_NO_EARLY) ? 0 : 1;
   g.wait_spins = ctx->dbg_wait_spins ? ctx->dbg_wait_spins : WAIT_SPINS; g.dbg_skip_kb = ctx->dbg_skip_kb;
   // Streamed K-major operands (more than 8 MB, i.e. not something that stays in L2 anyway) of the 3xTF32 kernels are
   // prefetched into L2 ahead of the loads: those kernels have only two or three stages in flight.  Measured on
   // 65 536 x 256 x 256: 3xTF32 A.B 65.0 -> 59.7 us, A.B^T 63.4 -> 59.3 us; the TF32 kernels (four or more stages)
   // and MN-major operands (one prefetch per 32-column box) got slower with it, so they do not use it.
   {
-    const bool pf_off = getenv("TALOS_TC_NO_PREFETCH") != nullptr;
+    const bool pf_off = (sw & SW_TC_NO_PREFETCH) != 0;
     g.pf_a = (!pf_off && x3 && !a_mn && (int64_t)M * K * g.batch > (2 << 20)) ? 1 : 0;
     g.pf_b = (!pf_off && x3 && !b_mn && (int64_t)N * K * g.batch > (2 << 20)) ? 1 : 0;
   }
@@ -526,11 +528,11 @@ void tc_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K
   // They also need enough 256 x 256 tiles to occupy every CTA pair without splitting K (the split-K weight-gradient
   // shapes have one or two tiles and are faster on 148 independent CTAs than on 74 pairs).
   const bool pair_shape = K >= 1024 && ceil_div(M, 2 * BM) * ceil_div(N, 256) >= ctx->sm_count / 2;
-  const bool pair = ctx->dbg_skip_kb < 0 && !batched && bn == 256 && M >= 256 && (pair_shape || g_check_pair || getenv("TALOS_TC_FORCE_PAIR")) && !getenv("TALOS_TC_NO_PAIR");
+  const bool pair = ctx->dbg_skip_kb < 0 && !batched && bn == 256 && M >= 256 && (pair_shape || g_check_pair || (sw & SW_TC_FORCE_PAIR)) && !(sw & SW_TC_NO_PAIR);
   g.m_tiles = (int)ceil_div(M, pair ? 2 * BM : BM); g.n_tiles = (int)ceil_div(N, bn); g.kb_total = (int)ceil_div(K, BK);
   // Groups of 8 row panels once there are enough tiles for the order to matter (with ~148 tiles in flight an 8-wide
   // group makes each wave touch 8 row panels and ~n/8 column panels instead of every row panel).
-  g.group_m = (g.m_tiles >= 16 && g.n_tiles >= 4 && !getenv("TALOS_TC_NO_RASTER")) ? 8 : g.m_tiles;
+  g.group_m = (g.m_tiles >= 16 && g.n_tiles >= 4 && !(sw & SW_TC_NO_RASTER)) ? 8 : g.m_tiles;
   int tiles = g.m_tiles * g.n_tiles, splits = 1;
   const int workers = pair ? ctx->sm_count / 2 : ctx->sm_count;   // CTAs, or CTA pairs
   // Split K when the output tiles alone cannot occupy the workers.  The tensor core truncates when it adds into the
@@ -544,11 +546,20 @@ void tc_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K
   // The one-CTA kernel, too, meets the chain cap on chip (a finished chain is folded into a running sum in the second
   // TMEM buffer), so an item may hold several chains: the 256 x 256 x 65 536 weight gradient then runs 2 x 74 items of 28
   // k-blocks (two chains) instead of 2 x 147 of 14, which halves the partial tiles the gather kernel has to add.
-  const bool fold_one = x3 && !batched && !pair && !getenv("TALOS_TC_NO_FOLD");
+  const bool fold_one = x3 && !batched && !pair && !(sw & SW_TC_NO_FOLD);
   g.kb_per_split = g.kb_total;
+  // What `s` slabs through memory cost, in k-blocks of this kernel's main loop (0.35 us per k-block of a 256-column tile in
+  // TF32, 1.4 us in 3xTF32): every slab is written and read once, from L2 while they fit beside the operands, and the
+  // reduction is one more launch.  65 536 x 256 x 1024 (the second feed-forward product) used to split in two to fill
+  // its last round: 172 us + 80 us of reduction, 186 us unsplit.
+  auto slab_cost = [&](int64_t s) {
+    if (s <= 1) return 0.0;
+    const double bytes = 8.0 * (double)s * (double)M * (double)N, kb_us = (x3 ? 1.4 : 0.35) * bn / 256.0;
+    return (bytes / (bytes > 64e6 ? 6.0e6 : 12.0e6) + 2.0) / kb_us;
+  };
   if (!batched && ((tiles * 2 <= workers && g.kb_total >= 16) || g.kb_total > cap)) {
     const int item_overhead = 3;
-    long long best_cost = -1;
+    double best_cost = -1;
     for (int r = 1; r <= 8; ++r) {
       const int s_r = (int)std::max<int64_t>(1, (int64_t)r * workers / tiles);
       int kps = (int)ceil_div(g.kb_total, s_r);
@@ -556,23 +567,22 @@ void tc_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K
       kps = std::max(kps, std::min(8, g.kb_total));
       if (kps > cap && !(fold_one && kps <= 8 * cap)) continue;
       const int chains = (int)ceil_div(kps, cap);
-      const long long cost = (long long)ceil_div((int64_t)tiles * ceil_div(g.kb_total, kps), workers) * (kps + item_overhead + (chains - 1));
+      const int64_t n_split = ceil_div(g.kb_total, kps);
+      const double cost = (double)ceil_div((int64_t)tiles * n_split, workers) * (kps + item_overhead + (chains - 1)) + slab_cost(n_split);
       if (best_cost < 0 || cost < best_cost) { best_cost = cost; g.kb_per_split = kps; }
     }
     if (g.kb_per_split > cap && !(fold_one && best_cost >= 0)) g.kb_per_split = cap;
   }
   if (g_check_fold && fold_one && g.kb_total > cap) g.kb_per_split = g.kb_total;
   g.chain_kb = (fold_one && g.kb_per_split > cap) ? cap : 0;
-  if (pair && x3 && g.kb_total > cap && !getenv("TALOS_TC_NO_FOLD")) {
+  if (pair && x3 && g.kb_total > cap && !(sw & SW_TC_NO_FOLD)) {
     // CTA-pair kernel: the chain cap is met ON CHIP (finished chains are folded into a running sum in TMEM), so K is
-    // split through memory only as far as it takes to keep the pairs busy: the smallest power-of-two split whose
-    // last round is at least 95 % full (4096^3: 2 slabs of 4 chains instead of 8 slabs through memory).
-    int best_s = 1; double best_eff = 0.0;
+    // split through memory only where filling the last round of pairs gains more than the slabs cost (4096^3: 2 slabs of
+    // 4 chains instead of 8 slabs through memory).
+    int best_s = 1; double best = -1.0;
     for (int s_ext = 1; s_ext <= 8 && g.kb_total / s_ext >= cap; s_ext *= 2) {
-      const int64_t n_items = (int64_t)tiles * s_ext, rounds = ceil_div(n_items, workers);
-      const double eff = (double)n_items / (double)(rounds * workers);
-      if (eff > best_eff + 0.03) { best_eff = eff; best_s = s_ext; }
-      if (eff >= 0.95) break;
+      const double cost = (double)ceil_div((int64_t)tiles * s_ext, workers) * (ceil_div(g.kb_total, s_ext) + 2) + slab_cost(s_ext);
+      if (best < 0 || cost < 0.97 * best) { best = cost; best_s = s_ext; }
     }
     g.kb_per_split = (int)(ceil_div(ceil_div(g.kb_total, best_s), cap) * cap);     // whole chains per item
     g.chain_kb = cap;
@@ -636,7 +646,7 @@ void tc_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K
   const bool aux_cfg = (aux_x3 || aux_tf32) && !batched && !a_mn && !b_mn && !pair && splits == 1 && g.n_tiles * (bn / 64) <= 4;
   const bool auxt = extra && extra->tanh_saved && extra->colsum_part && extra->colsum_slabs_out && aux_cfg && !(N & 31) && plain_epi && g.tma_out &&
                     !(((uintptr_t)extra->tanh_saved) & 15) && !(extra->ld_saved & 3) && extra->colsum_floats >= (size_t)4 * grid * N &&
-                    !getenv("TALOS_TC_NO_FUSED_DACT");
+                    !(sw & SW_TC_NO_FUSED_DACT);
   CUtensorMap tx = tc;
   if (auxt) ok = ok && make_out_tmap(&tx, extra->tanh_saved, 1, M, N, extra->ld_saved, M * extra->ld_saved);
   TALOS_REQUIRE(ok, TALOS_ERR_CUDA, "cuTensorMapEncodeTiled failed");
@@ -644,7 +654,8 @@ void tc_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K
     g.colsum_part = extra->colsum_part;
 #define TALOS_TC_AUX(BNv, ST, X3v, SB, EWv)                                                                                         \
   { const size_t smem = tc_smem_bytes<BNv, ST, X3v, SB, EWv>() + 128;                                                               \
-    TALOS_CHECK_CUDA(cudaFuncSetAttribute(gemm_tc_aux_kernel<BNv, ST, X3v, SB, EWv>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+    static std::atomic<uint64_t> smem_set{0};                                                                                       \
+    talos_allow_smem(smem_set, (const void*)gemm_tc_aux_kernel<BNv, ST, X3v, SB, EWv>, smem, ctx->device);                          \
     gemm_tc_aux_kernel<BNv, ST, X3v, SB, EWv><<<grid, TcRoles<X3v, X3v, BNv, EWv>::THREADS, smem, ctx->stream>>>(ta, tb, tc, tbl, tx, g); }
     if (!x3) TALOS_TC_AUX(256, 3, false, 2, 0)
     else if (bn == 128 && wide_epi) TALOS_TC_AUX(128, 2, true, 1, 16)
@@ -664,7 +675,7 @@ void tc_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K
 #define TALOS_TC_CASE(BNv, ST, SB, ST3, SB3)                                                                      \
   if (bn == BNv) {                                                                                                \
     if (x3 && presplit) launch_major<BNv, ST3, true, 1, true, SB3>(ctx, a_mn, b_mn, ta, tb, tc, tbl, g, grid);    \
-    else if (x3 && BNv == 256 && !getenv("TALOS_TC_NO_EPI8")) launch_major<BNv, ST3, true, 1, false, SB3, (BNv == 256 ? 8 : 0)>(ctx, a_mn, b_mn, ta, tb, tc, tb, g, grid); \
+    else if (x3 && BNv == 256 && !(sw & SW_TC_NO_EPI8)) launch_major<BNv, ST3, true, 1, false, SB3, (BNv == 256 ? 8 : 0)>(ctx, a_mn, b_mn, ta, tb, tc, tb, g, grid); \
     else if (x3) launch_major<BNv, ST3, true, 1, false, SB3>(ctx, a_mn, b_mn, ta, tb, tc, tb, g, grid);           \
     else launch_major<BNv, ST, false, 1, false, SB>(ctx, a_mn, b_mn, ta, tb, tc, tb, g, grid);                    \
   }
@@ -747,7 +758,7 @@ bool self_check(talos_ctx* ctx) {
 
 static bool tc_ready(talos_ctx* ctx) {
   if (ctx->tc_state < 0) return false;
-  if (getenv("TALOS_DISABLE_TENSOR_CORES")) return false;
+  if (talos_switches() & SW_DISABLE_TENSOR_CORES) return false;
   if (ctx->tc_state == 0) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(ctx->stream, &cap);
@@ -769,9 +780,13 @@ bool talos_gemm_tc_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N
                           const float* B, int64_t ldb, float* C, int64_t ldc, int mode, const EpiArgs& epi, const TcExtra* extra) {
   if (extra && extra->splits_out) *extra->splits_out = 1;
   if (ctx->tc_state < 0) return false;
-  // TMA needs 16-byte aligned bases and row pitches; tiny problems are launch-bound and stay on CUDA cores.
+  // TMA needs 16-byte aligned bases and row pitches.  Problems below 2^26 products are launch-bound here (operand
+  // preparation + tiles that fill a few SMs: 11 to 25 us) and stay on the CUDA cores (gemm_small.cu: 512 x 64 x 64 11.3 -> 4.2 us,
+  // 512 x 256 x 256 24.6 -> 10.3, 4 096 x 64 x 256 even) unless their reduction is long or the caller brings prepared
+  // weights or a fused epilogue.
   if ((((uintptr_t)A | (uintptr_t)B) & 15) || (lda & 3) || (ldb & 3) || K < 1) return false;
-  if (M * N * K < (1LL << 18) || M < 1 || N < 1) return false;
+  const bool small_ok = !extra && K <= 4096 && !(talos_switches() & SW_TC_NO_SMALL);
+  if (M * N * K < (small_ok ? 1LL << 26 : 1LL << 18) || M < 1 || N < 1) return false;
   if (!tc_ready(ctx)) return false;
   if (extra && extra->b_hi && ((((uintptr_t)extra->b_hi | (uintptr_t)extra->b_lo) & 15) != 0)) return false;
   tc_launch(ctx, opA, opB, M, N, K, A, lda, B, ldb, C, ldc, mode, epi, TcBatch{1, 0, 0, 0}, extra);

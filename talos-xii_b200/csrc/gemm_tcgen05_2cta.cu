@@ -255,7 +255,8 @@ template <int BN, int STAGES, bool X3, bool A_MN, bool B_MN, bool BPS>
 void launch2_one(talos_ctx* ctx, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tbl, const TcArgs& g, int grid) {
   auto kern = gemm_tc2_kernel<BN, STAGES, X3, A_MN, B_MN, BPS>;
   size_t smem = tc2_smem_bytes<BN, STAGES, X3>();
-  TALOS_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static std::atomic<uint64_t> smem_set{0};
+  talos_allow_smem(smem_set, (const void*)kern, smem, ctx->device);
   kern<<<grid, X3 ? 448 : 320, smem, ctx->stream>>>(ta, tb, tc, tbl, g);
   talos_launched(ctx, "gemm_tcgen05_2cta");
 }

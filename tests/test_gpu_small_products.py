@@ -1,0 +1,83 @@
+"""The small-product kernels (gemm_small.cu) at the sizes where they can go wrong: tile edges (16, 32 and 64 wide), K around
+a chunk (128) and around what a cluster splits, widths that rule out 128-bit accesses, every operand layout, and the
+one-launch Linear backward with its fused activation derivative and bias gradient.  The reference is float64; fp32 sums of K
+terms with round-to-nearest products stay within sqrt(K) * 2^-23 of it in the 2-norm, 1e-5 allows a factor of ten at K = 1 100."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from gpu_util import dev, host, normal, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx(talos):
+    c = talos.torch_context(0)
+    yield c
+    c.synchronize()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (15, 17, 5), (16, 16, 128), (33, 31, 129), (64, 64, 64), (65, 4, 300), (40, 36, 1100), (1000, 64, 20),
+                                   (2100, 68, 33), (17, 2000, 8), (200, 200, 1025)])
+@pytest.mark.parametrize("opA,opB", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_product(talos, ctx, M, N, K, opA, opB):
+    import torch
+    A, B = normal(1, (K, M) if opA else (M, K)), normal(2, (N, K) if opB else (K, N))
+    bias, C0 = normal(3, (N,)), normal(4, (M, N))
+    a, b, bi, c = dev(A), dev(B), dev(bias), dev(np.pad(C0, ((0, 1), (0, 0)), constant_values=-7.0))
+    epi = talos.Epilogue(bias=talos.ptr(bi), act=talos.ACT_TANH, beta=1)
+    talos.lib.talos_gemm(ctx.handle, opA, opB, M, N, K, talos.ptr(a), A.shape[1], talos.ptr(b), B.shape[1], talos.ptr(c), N, 1, ctypes.byref(epi))
+    ref = C0 + np.tanh((A.T if opA else A) @ (B.T if opB else B) + bias)
+    got = host(c)
+    assert rel_err(got[:M], ref) <= 1e-5
+    assert np.all(got[M] == -7.0)                                # nothing past the last row
+
+
+@pytest.mark.parametrize("rows,fin,fout", [(1, 1, 1), (64, 8, 64), (64, 64, 1), (64, 64, 5), (129, 12, 20), (300, 64, 64), (1100, 7, 33), (4096, 8, 16), (500, 256, 256)])
+@pytest.mark.parametrize("act", ["none", "tanh", "relu", "silu"])
+@pytest.mark.parametrize("parts", ["all", "dx", "dw", "accumulate"])
+def test_linear_backward(talos, ctx, rows, fin, fout, act, parts):
+    import torch
+    x, W, saved, dy = normal(5, (rows, fin)), normal(6, (fin, fout)), np.tanh(normal(7, (rows, fout))), normal(8, (rows, fout))
+    saved = saved.astype(np.float32).astype(np.float64)
+    if act == "none": d = 1.0
+    elif act == "tanh": d = 1 - saved ** 2
+    elif act == "relu": d = (saved > 0).astype(np.float64)
+    else:
+        g = 1 / (1 + np.exp(-saved)); d = g * (1 + saved * (1 - g))
+    dz = dy * d
+    acc = 7 if parts == "accumulate" else 0
+    base = [normal(9, (rows, fin)), normal(10, (fin, fout)), normal(11, (fout,))]
+    out = [dev(np.append(b.ravel(), -7.0)) for b in base]
+    tx, tw, ts, ty = dev(x), dev(W), dev(saved), dev(dy)
+    want = [parts != "dw", parts != "dx", parts != "dx"]
+    talos.lib.talos_linear_bwd(ctx.handle, talos.ptr(tx), talos.ptr(tw), talos.ptr(ts), talos.ptr(ty), *[talos.ptr(o) if w else None for o, w in zip(out, want)],
+                               rows, fin, fout, talos.ACTS[act], 1, acc)
+    ref = [dz @ W.T, x.T @ dz, dz.sum(0)]
+    for o, r, b, w in zip(out, ref, base, want):
+        got = host(o)
+        assert got[-1] == -7.0
+        if w:
+            # the column sum of N(0, 1)-sized terms can be far smaller than its terms: their own size is part of the bound
+            r = r + b if acc else r
+            err = np.linalg.norm(got[:-1].reshape(r.shape) - r)
+            assert err <= 1e-5 * max(np.linalg.norm(r), np.sqrt(r.size)), (err, np.linalg.norm(r))
+        else:
+            assert np.array_equal(got[:-1], b.ravel().astype(np.float32))
+
+
+@pytest.mark.needs_tensor_cores
+@pytest.mark.parametrize("mode", [1, 2])
+@pytest.mark.parametrize("M,N,K", [(200, 72, 40), (129, 33, 100), (1000, 36, 520), (64, 260, 64)])
+def test_both_routes_of_a_small_product(talos, ctx, M, N, K, mode, monkeypatch):
+    # the tensor-core kernels stay in use for products of this size that bring prepared weights (the PPO trainer's)
+    import torch
+    A, B = normal(12, (M, K)), normal(13, (K, (N + 3) // 4 * 4))
+    a, b, c = dev(A), dev(B), torch.empty(M, N, device="cuda:0")
+    for route, tol in (("small", 1e-5), ("tensor", 1e-5 if mode == 1 else 2e-3)):
+        if route == "tensor":
+            monkeypatch.setenv("TALOS_TC_NO_SMALL", "1")
+        talos.lib.talos_gemm(ctx.handle, 0, 0, M, N, K, talos.ptr(a), K, talos.ptr(b), B.shape[1], talos.ptr(c), N, mode, None)
+        assert rel_err(c, A @ B[:, :N]) <= tol, route

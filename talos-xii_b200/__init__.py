@@ -9,12 +9,15 @@ binding cannot drift from the ABI.  A non-zero status raises `TalosError` carryi
 no CPU path: loading the library or creating a context without a CUDA device fails loudly.
 """
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 import re
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 INCLUDE_DIR = os.path.join(os.path.dirname(_HERE), "include")
 LIB_PATH = os.path.join(_HERE, "libtalos_b200.so")
+BINDING_PATH = os.path.join(_HERE, "_pycall.so")
 
 OK, ERR_ARG, ERR_SHAPE, ERR_ALLOC, ERR_CUDA, ERR_NCCL, ERR_TIMEOUT, ERR_UNSUPPORTED = range(8)
 MODE_FP32, MODE_TF32X3, MODE_TF32 = 0, 1, 2
@@ -81,8 +84,19 @@ def parse_headers(include_dir=INCLUDE_DIR):
     return protos
 
 
+def _load_binding():
+    """The native call path (host/pycall.cpp): the same functions with the argument conversion compiled in."""
+    if not os.path.exists(BINDING_PATH):
+        raise ImportError("_pycall.so is not built; run `python talos-xii_b200/build.py`")
+    loader = importlib.machinery.ExtensionFileLoader("_pycall", BINDING_PATH)
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_pycall", BINDING_PATH, loader=loader))
+    loader.exec_module(mod)
+    return mod
+
+
 class _Lib:
-    """Attribute access gives a checked callable: status != 0 raises TalosError."""
+    """Attribute access gives a checked callable: status != 0 raises TalosError.  Calls with plain arguments (ints,
+    floats, None, context handles) take the native path, all others the ctypes function."""
 
     def __init__(self):
         if not os.path.exists(LIB_PATH):
@@ -93,6 +107,8 @@ class _Lib:
         for name, (restype, argtypes) in self.protos.items():
             f = getattr(self.cdll, name)
             f.restype, f.argtypes = restype, argtypes
+        self.native, self.by_ctypes = _load_binding(), {}
+        self.native.setup(TalosError, C.c_void_p, self.by_ctypes)
 
     def raw(self, name):
         return getattr(self.cdll, name)
@@ -110,8 +126,9 @@ class _Lib:
             if st != 0:
                 raise TalosError(st, self.cdll.talos_last_error_string().decode())
         checked.__name__ = name
-        self.__dict__[name] = checked
-        return checked
+        self.by_ctypes[name] = checked
+        self.__dict__[name] = getattr(self.native, name)
+        return self.__dict__[name]
 
 
 _NOT_STATUS = {"talos_ctx_tensor_cores_active", "talos_ctx_tensor_cores_state", "talos_comm_peer_exchange_active"}

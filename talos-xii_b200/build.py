@@ -6,11 +6,13 @@ import concurrent.futures as cf
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libtalos_b200.so")
+BINDING = os.path.join(HERE, "_pycall.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--use_fast_math=false",
          "-Xcompiler", "-fPIC,-fvisibility=hidden,-Wall", "-Xptxas", "-v"]
@@ -55,7 +57,22 @@ def build(force=False, verbose=False):
         r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
         if r.returncode != 0:
             raise RuntimeError("link failed:\n" + r.stdout)
+    build_binding()
     return LIB
+
+
+def build_binding():
+    """Compiles the native call path of the Python binding (host/pycall.cpp) against the built library."""
+    src = os.path.join(HERE, "host", "pycall.cpp")
+    hdrs = [os.path.join(HERE, "..", "include", h) for h in ("talos_b200.h", "talos_b200_ppo.h")]
+    if os.path.exists(BINDING) and os.path.getmtime(BINDING) > max(os.path.getmtime(f) for f in [src, LIB] + hdrs):
+        return BINDING
+    cmd = ["g++", "-std=c++17", "-O2", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden", "-I", sysconfig.get_paths()["include"], "-o", BINDING, src,
+           "-L", HERE, "-ltalos_b200", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed for pycall.cpp:\n" + r.stdout)
+    return BINDING
 
 
 def build_host_tests():

@@ -15,6 +15,7 @@ template <int TS>
 __global__ void __launch_bounds__(256)
 attention_fwd_kernel(HeadView q1, HeadView q2, HeadView k1, HeadView k2, HeadView v, HeadViewOut out, float* probs,
                      int H, int S, float scale, int causal) {
+  talos_pdl(probs);
   extern __shared__ float sm[];
   const int dqk = q1.d + q2.d, dv = v.d, SP = S + 1;
   float* Qs = sm;                       // [S][dqk]
@@ -119,7 +120,7 @@ void talos_attention_launch(talos_ctx* ctx, HeadView q1, HeadView q2, HeadView k
   const int ts = (S + 15) / 16;
   auto launch = [&](auto kern) {
     TALOS_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem));
-    kern<<<(unsigned)(B * H), 256, shmem, ctx->stream>>>(q1, q2, k1, k2, v, out, probs, H, S, scale, causal);
+    talos_kernel(ctx, kern, (unsigned)(B * H), 256, shmem, q1, q2, k1, k2, v, out, probs, H, S, scale, causal);
   };
   if (ts <= 1) launch(attention_fwd_kernel<1>);
   else if (ts <= 2) launch(attention_fwd_kernel<2>);

@@ -80,6 +80,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   }
   if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
+  talos_pdl();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
@@ -262,7 +263,7 @@ bool talos_attention_tc_fused(talos_ctx* ctx, const float* q, const float* k, co
   static std::atomic<uint64_t> smem_set{0};
   talos_allow_smem(smem_set, (const void*)attention_tc_kernel, 227 * 1024, ctx->device);
   const int grid = (int)std::min<int64_t>(BH, ctx->sm_count);
-  attention_tc_kernel<<<grid, ATT_THREADS, smem, ctx->stream>>>(tq, tk, tv, to, tp, g);
+  talos_kernel(ctx, attention_tc_kernel, grid, ATT_THREADS, smem, tq, tk, tv, to, tp, g);
   talos_launched(ctx, "attention_tc_fused");
   return true;
 }

@@ -42,6 +42,7 @@ float* scratch_for_current_device(int device) {
 // Stage 1: CTA `s` sums rows [s*rows_per, (s+1)*rows_per) of every column into scratch[s][*].
 __global__ void static_colsum_stage1(const float* __restrict__ g, long long rows, int n, long long rows_per,
                                      float* __restrict__ scratch) {
+  talos_pdl(g, scratch);
   const long long r0 = (long long)blockIdx.x * rows_per, r1 = min(rows, r0 + rows_per);
   for (int c = threadIdx.x; c < n; c += blockDim.x) {
     float s = 0.f;
@@ -52,6 +53,7 @@ __global__ void static_colsum_stage1(const float* __restrict__ g, long long rows
 }
 // Stage 2: one thread per column adds the slab sums in slab order.
 __global__ void static_colsum_stage2(const float* __restrict__ scratch, int slabs, int n, float* __restrict__ out, int acc) {
+  talos_pdl(scratch, out);
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   float s = 0.f;
@@ -82,9 +84,9 @@ TALOS_API talos_status talos_colsum_noalloc(talos_ctx* ctx, const float* g, floa
   slabs = std::max<int64_t>(1, ceil_div(rows, rows_per));
   // Stage 1 overwrites every scratch element stage 2 reads (slabs x n), so nothing left over from an earlier
   // call is ever consumed and nothing needs clearing.
-  static_colsum_stage1<<<(unsigned)slabs, 256, 0, ctx->stream>>>(g, rows, (int)n, rows_per, scratch);
+  talos_kernel(ctx, static_colsum_stage1, (unsigned)slabs, 256, 0, g, rows, (int)n, rows_per, scratch);
   talos_launched(ctx, "colsum_noalloc_stage1");
-  static_colsum_stage2<<<(unsigned)ceil_div(n, 128), 128, 0, ctx->stream>>>(scratch, (int)slabs, (int)n, out, accumulate ? 1 : 0);
+  talos_kernel(ctx, static_colsum_stage2, (unsigned)ceil_div(n, 128), 128, 0, scratch, (int)slabs, (int)n, out, accumulate ? 1 : 0);
   talos_launched(ctx, "colsum_noalloc_stage2");
   TALOS_ENTRY_END
 }

@@ -32,6 +32,7 @@ mla_decode_kernel(const float* __restrict__ q_c, const float* __restrict__ q_r, 
                   const float* __restrict__ k_r, const float* __restrict__ v_c, const float* __restrict__ cos_t,
                   const float* __restrict__ sin_t, long long table_len, const int* __restrict__ pos, float* k_cache,
                   float* v_cache, float* __restrict__ out, long long items, int H, int dh, int dr, int cap, float scale) {
+  talos_pdl(q_c, q_r, k_c, k_r, v_c, cos_t, sin_t, pos, k_cache, v_cache, out);
   extern __shared__ __align__(16) float dec_sm[];
   const int dk = dh + dr, dk_pad = (dk + 3) & ~3, cap_pad = (cap + 3) & ~3;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -96,6 +97,7 @@ mla_decode_kernel(const float* __restrict__ q_c, const float* __restrict__ q_r, 
 }
 
 __global__ void decode_advance_kernel(int* pos, const int* __restrict__ reset, long long n) {
+  talos_pdl(pos, reset);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) pos[i] = (reset && reset[i]) ? 0 : pos[i] + 1;
 }
@@ -119,10 +121,10 @@ TALOS_API talos_status talos_mla_decode_step(talos_ctx* ctx, const float* q_c, c
   const unsigned grid = (unsigned)ceil_div(items, DEC_WARPS);
   const bool vec = (dk % 4 == 0) && (((uintptr_t)k_cache & 15) == 0);
   if (vec)
-    mla_decode_kernel<true><<<grid, DEC_WARPS * 32, shmem, ctx->stream>>>(q_c, q_r, k_c, k_r, v_c, cos_t, sin_t, table_len, pos, k_cache, v_cache, out,
+    talos_kernel(ctx, mla_decode_kernel<true>, grid, DEC_WARPS * 32, shmem, q_c, q_r, k_c, k_r, v_c, cos_t, sin_t, table_len, pos, k_cache, v_cache, out,
                                                                           items, (int)H, (int)dh, (int)dr, (int)cap, scale);
   else
-    mla_decode_kernel<false><<<grid, DEC_WARPS * 32, shmem, ctx->stream>>>(q_c, q_r, k_c, k_r, v_c, cos_t, sin_t, table_len, pos, k_cache, v_cache, out,
+    talos_kernel(ctx, mla_decode_kernel<false>, grid, DEC_WARPS * 32, shmem, q_c, q_r, k_c, k_r, v_c, cos_t, sin_t, table_len, pos, k_cache, v_cache, out,
                                                                            items, (int)H, (int)dh, (int)dr, (int)cap, scale);
   talos_launched(ctx, "mla_decode_step");
   TALOS_ENTRY_END
@@ -134,7 +136,7 @@ TALOS_API talos_status talos_decode_advance(talos_ctx* ctx, int32_t* pos, const 
   TALOS_REQUIRE(N >= 0, TALOS_ERR_SHAPE, "bad count");
   if (N == 0) return TALOS_OK;
   TALOS_REQUIRE(pos, TALOS_ERR_ARG, "null pointer");
-  decode_advance_kernel<<<(unsigned)ceil_div(N, 256), 256, 0, ctx->stream>>>(pos, reset, N);
+  talos_kernel(ctx, decode_advance_kernel, (unsigned)ceil_div(N, 256), 256, 0, pos, reset, N);
   talos_launched(ctx, "decode_advance");
   TALOS_ENTRY_END
 }

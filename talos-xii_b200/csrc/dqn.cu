@@ -7,6 +7,7 @@ namespace {
 
 // q[b][a] = v[b] + adv[b][a] - mean_a(adv[b][:])                     (src/dqn.rs:76-93: the three matmuls with ones)
 __global__ void dueling_fwd_kernel(const float* __restrict__ v, const float* __restrict__ adv, float* __restrict__ q, long long B, int A) {
+  talos_pdl(v, adv, q);
   const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= B) return;
   float s = 0.f;
@@ -16,6 +17,7 @@ __global__ void dueling_fwd_kernel(const float* __restrict__ v, const float* __r
 }
 // dv[b] (+)= sum_a dq[b][a];  dadv[b][a] (+)= dq[b][a] - mean_a(dq[b][:])
 __global__ void dueling_bwd_kernel(const float* __restrict__ dq, float* __restrict__ dv, float* __restrict__ dadv, long long B, int A, int acc) {
+  talos_pdl(dq, dv, dadv);
   const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= B) return;
   float s = 0.f;
@@ -30,6 +32,7 @@ __global__ void dueling_bwd_kernel(const float* __restrict__ dq, float* __restri
 // network values it: target[b] = r[b] + gamma * Qt[b][argmax_a Qe[b][a]] * (1 - done[b]).
 __global__ void dqn_target_kernel(const float* __restrict__ q_eval, const float* __restrict__ q_target, const float* __restrict__ rewards,
                                   const float* __restrict__ dones, float gamma, float* __restrict__ target, long long B, int A) {
+  talos_pdl(q_eval, q_target, rewards, dones, target);
   const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= B) return;
   int best = 0; float mx = -INFINITY;
@@ -42,6 +45,7 @@ __global__ void dqn_target_kernel(const float* __restrict__ q_eval, const float*
 __global__ void __launch_bounds__(256)
 dqn_loss_kernel(const float* __restrict__ q, const int32_t* __restrict__ actions, const float* __restrict__ target, float* __restrict__ loss,
                 float* __restrict__ dq, long long B, int A, int32_t* __restrict__ status) {
+  talos_pdl(q, actions, target, loss, dq, status);
   __shared__ double sh[256];
   double acc = 0.0;
   for (long long b = threadIdx.x; b < B; b += 256) {
@@ -61,6 +65,7 @@ dqn_loss_kernel(const float* __restrict__ q, const int32_t* __restrict__ actions
 }
 // target <- target * (1 - tau) + source * tau                           (src/dqn.rs:129-150)
 __global__ void soft_update_kernel(float* __restrict__ t, const float* __restrict__ s, float tau, long long n) {
+  talos_pdl(t, s);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) t[i] = t[i] * (1.f - tau) + s[i] * tau;
 }
@@ -73,7 +78,7 @@ TALOS_API talos_status talos_dueling_combine_fwd(talos_ctx* ctx, const float* v,
   TALOS_REQUIRE(B >= 0 && A >= 1 && A <= 4096, TALOS_ERR_SHAPE, "bad dueling shape");
   if (B == 0) return TALOS_OK;
   TALOS_REQUIRE(v && adv && q, TALOS_ERR_ARG, "null pointer");
-  dueling_fwd_kernel<<<(unsigned)ceil_div(B, 128), 128, 0, ctx->stream>>>(v, adv, q, B, (int)A);
+  talos_kernel(ctx, dueling_fwd_kernel, (unsigned)ceil_div(B, 128), 128, 0, v, adv, q, B, (int)A);
   talos_launched(ctx, "dueling_fwd");
   TALOS_ENTRY_END
 }
@@ -84,7 +89,7 @@ TALOS_API talos_status talos_dueling_combine_bwd(talos_ctx* ctx, const float* dq
   TALOS_REQUIRE(B >= 0 && A >= 1 && A <= 4096, TALOS_ERR_SHAPE, "bad dueling shape");
   if (B == 0) return TALOS_OK;
   TALOS_REQUIRE(dq && (dv || dadv), TALOS_ERR_ARG, "null pointer");
-  dueling_bwd_kernel<<<(unsigned)ceil_div(B, 128), 128, 0, ctx->stream>>>(dq, dv, dadv, B, (int)A, accumulate ? 1 : 0);
+  talos_kernel(ctx, dueling_bwd_kernel, (unsigned)ceil_div(B, 128), 128, 0, dq, dv, dadv, B, (int)A, accumulate ? 1 : 0);
   talos_launched(ctx, "dueling_bwd");
   TALOS_ENTRY_END
 }
@@ -96,7 +101,7 @@ TALOS_API talos_status talos_dqn_target(talos_ctx* ctx, const float* q_next_eval
   TALOS_REQUIRE(B >= 0 && A >= 1 && A <= 4096, TALOS_ERR_SHAPE, "bad DQN target shape");
   if (B == 0) return TALOS_OK;
   TALOS_REQUIRE(q_next_eval && q_next_target && rewards && dones && target, TALOS_ERR_ARG, "null pointer");
-  dqn_target_kernel<<<(unsigned)ceil_div(B, 128), 128, 0, ctx->stream>>>(q_next_eval, q_next_target, rewards, dones, gamma, target, B, (int)A);
+  talos_kernel(ctx, dqn_target_kernel, (unsigned)ceil_div(B, 128), 128, 0, q_next_eval, q_next_target, rewards, dones, gamma, target, B, (int)A);
   talos_launched(ctx, "dqn_target");
   TALOS_ENTRY_END
 }
@@ -107,7 +112,7 @@ TALOS_API talos_status talos_dqn_loss_fwd_bwd(talos_ctx* ctx, const float* q, co
   talos_check_ctx(ctx);
   TALOS_REQUIRE(B >= 1 && A >= 1 && A <= 4096, TALOS_ERR_SHAPE, "bad DQN loss shape");
   TALOS_REQUIRE(q && actions && target && loss, TALOS_ERR_ARG, "null pointer");
-  dqn_loss_kernel<<<1, 256, 0, ctx->stream>>>(q, actions, target, loss, dq, B, (int)A, ctx->dev_status);
+  talos_kernel(ctx, dqn_loss_kernel, 1, 256, 0, q, actions, target, loss, dq, B, (int)A, ctx->dev_status);
   talos_launched(ctx, "dqn_loss");
   TALOS_ENTRY_END
 }
@@ -118,7 +123,7 @@ TALOS_API talos_status talos_soft_update(talos_ctx* ctx, float* target_params, c
   TALOS_REQUIRE(n >= 0, TALOS_ERR_SHAPE, "bad length");
   if (n == 0) return TALOS_OK;
   TALOS_REQUIRE(target_params && source_params, TALOS_ERR_ARG, "null pointer");
-  soft_update_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, ctx->stream>>>(target_params, source_params, tau, n);
+  talos_kernel(ctx, soft_update_kernel, (unsigned)ceil_div(n, 256), 256, 0, target_params, source_params, tau, n);
   talos_launched(ctx, "soft_update");
   TALOS_ENTRY_END
 }

@@ -23,6 +23,7 @@ struct SwapArgs { FastDiv run, dlo, mid, dhi; unsigned s_o, s_i, s_m, s_j; };   
 template <typename V>
 __global__ void __launch_bounds__(256)
 swap_axes_kernel(const V* __restrict__ x, V* __restrict__ y, unsigned n, SwapArgs a) {
+  talos_pdl(x, y);
   V v[4];
   const unsigned first = blockIdx.x * 1024 + threadIdx.x;
 #pragma unroll
@@ -45,6 +46,7 @@ struct TransposeArgs { long long in_stride[6]; long long out_shape[6]; int rank;
 // General axis swap.  Each thread produces one output element; when the innermost axis is
 // untouched the innermost index is contiguous on both sides, so loads and stores coalesce.
 __global__ void transpose_kernel(const float* __restrict__ x, float* __restrict__ y, long long n, TransposeArgs a, int acc) {
+  talos_pdl(x, y);
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n) return;
   long long rem = idx, src = 0;
@@ -58,6 +60,7 @@ __global__ void transpose_kernel(const float* __restrict__ x, float* __restrict_
 
 // 2-D tiled transpose of the two innermost axes ([batch, R, C] -> [batch, C, R]) through shared memory.
 __global__ void transpose2d_kernel(const float* __restrict__ x, float* __restrict__ y, int R, int Cc, int acc) {
+  talos_pdl(x, y);
   __shared__ float tile[32][33];
   const float* xb = x + (long long)blockIdx.z * R * Cc; float* yb = y + (long long)blockIdx.z * R * Cc;
   int c = blockIdx.x * 32 + threadIdx.x, r0 = blockIdx.y * 32;
@@ -72,6 +75,7 @@ __global__ void transpose2d_kernel(const float* __restrict__ x, float* __restric
 
 __global__ void concat_last_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out,
                                    long long rows, int da, int db) {
+  talos_pdl(a, b, out);
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   int w = da + db; if (idx >= rows * w) return;
   long long r = idx / w; int c = (int)(idx % w);
@@ -79,6 +83,7 @@ __global__ void concat_last_kernel(const float* __restrict__ a, const float* __r
 }
 __global__ void split_last_kernel(const float* __restrict__ g, float* __restrict__ ga, float* __restrict__ gb,
                                   long long rows, int da, int db, int acc) {
+  talos_pdl(g, ga, gb);
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   int w = da + db; if (idx >= rows * w) return;
   long long r = idx / w; int c = (int)(idx % w); float v = g[idx];
@@ -89,6 +94,7 @@ __global__ void split_last_kernel(const float* __restrict__ g, float* __restrict
 // HBM: splitting [65536, 768] into 256 | 512 160 -> 62 us.
 __global__ void __launch_bounds__(256)
 concat_last_vec_kernel(const float4* __restrict__ a, const float4* __restrict__ b, float4* __restrict__ out, unsigned n, FastDiv width, unsigned da) {
+  talos_pdl(a, b, out);
   const unsigned first = blockIdx.x * 1024 + threadIdx.x, db = width.d - da;
   float4 v[4];
 #pragma unroll
@@ -101,6 +107,7 @@ concat_last_vec_kernel(const float4* __restrict__ a, const float4* __restrict__ 
 }
 __global__ void __launch_bounds__(256)
 split_last_vec_kernel(const float4* __restrict__ g, float4* __restrict__ ga, float4* __restrict__ gb, unsigned n, FastDiv width, unsigned da, int acc) {
+  talos_pdl(g, ga, gb);
   const unsigned first = blockIdx.x * 1024 + threadIdx.x, db = width.d - da;
   float4 v[4];
 #pragma unroll
@@ -117,12 +124,14 @@ split_last_vec_kernel(const float4* __restrict__ g, float4* __restrict__ ga, flo
   }
 }
 __global__ void last_token_kernel(const float* __restrict__ x, float* __restrict__ y, long long B, long long S, int D) {
+  talos_pdl(x, y);
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= B * D) return;
   long long b = idx / D; int d = (int)(idx % D);
   y[idx] = x[(b * S + (S - 1)) * D + d];
 }
 __global__ void bias_add_kernel(float* __restrict__ y, const float* __restrict__ bias, long long total, int n) {
+  talos_pdl(y, bias);
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx < total) y[idx] += __ldg(bias + (idx % n));
 }
@@ -162,11 +171,13 @@ __device__ __forceinline__ float ew_bwd(int op, float x, float p0, float p1) {
   }
 }
 __global__ void ew_unary_kernel(int op, const float* __restrict__ x, float* __restrict__ y, long long n, float p0, float p1) {
+  talos_pdl(x, y);
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] = ew_fwd(op, x[i], p0, p1);
 }
 __global__ void ew_unary_bwd_kernel(int op, const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ dx,
                                     long long n, float p0, float p1) {
+  talos_pdl(x, dy, dx);
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dx[i] += dy[i] * ew_bwd(op, x[i], p0, p1);
 }
@@ -179,6 +190,7 @@ __device__ __forceinline__ float ew_binary(int op, float u, float v) {
 template <typename V>
 __global__ void __launch_bounds__(256)
 ew_binary_kernel(int op, const V* a, const V* b, V* y, long long n, int rest) {
+  talos_pdl(a, b, y);
   if (rest && blockIdx.x == gridDim.x - 1) {
     const float *at = (const float*)(a + n), *bt = (const float*)(b + n); float* yt = (float*)(y + n);
     if ((int)threadIdx.x < rest) yt[threadIdx.x] = ew_binary(op, at[threadIdx.x], bt[threadIdx.x]);
@@ -199,6 +211,7 @@ ew_binary_kernel(int op, const V* a, const V* b, V* y, long long n, int rest) {
 }
 // da/db may alias (x op x): both contributions are then added by the same thread in turn.
 __global__ void ew_binary_bwd_kernel(int op, const float* a, const float* b, const float* __restrict__ dy, float* da, float* db, long long n) {
+  talos_pdl(a, b, dy, da, db);
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float g = dy[i], u = a[i], v = b[i], ga, gb;
@@ -214,6 +227,7 @@ __global__ void ew_binary_bwd_kernel(int op, const float* a, const float* b, con
 
 // Deterministic sum: fixed grid, fixed per-thread order, second stage sums block partials in order.
 __global__ void reduce_stage1_kernel(const float* __restrict__ x, long long n, float* __restrict__ partial) {
+  talos_pdl(x, partial);
   __shared__ float sh[256];
   float s = 0.f;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) s += x[i];
@@ -222,6 +236,7 @@ __global__ void reduce_stage1_kernel(const float* __restrict__ x, long long n, f
   if (threadIdx.x == 0) partial[blockIdx.x] = sh[0];
 }
 __global__ void reduce_stage2_kernel(const float* __restrict__ partial, int nparts, float scale, float* out, int acc) {
+  talos_pdl(partial, out);
   __shared__ float sh[256];
   float s = 0.f;
   for (int i = threadIdx.x; i < nparts; i += 256) s += partial[i];
@@ -230,6 +245,7 @@ __global__ void reduce_stage2_kernel(const float* __restrict__ partial, int npar
   if (threadIdx.x == 0) out[0] = acc ? out[0] + sh[0] * scale : sh[0] * scale;
 }
 __global__ void fill_from_scalar_kernel(const float* __restrict__ s, float scale, float* __restrict__ y, long long n, int acc) {
+  talos_pdl(s, y);
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) { float v = s[0] * scale; y[i] = acc ? y[i] + v : v; }
 }
@@ -252,7 +268,7 @@ TALOS_API talos_status talos_transpose(talos_ctx* ctx, const float* x, float* y,
     int64_t batch = n / (shape[lo] * shape[hi]);
     if (batch <= 65535) {
       dim3 grid((unsigned)ceil_div(shape[hi], 32), (unsigned)ceil_div(shape[lo], 32), (unsigned)batch);
-      transpose2d_kernel<<<grid, dim3(32, 8), 0, ctx->stream>>>(x, y, (int)shape[lo], (int)shape[hi], accumulate ? 1 : 0);
+      talos_kernel(ctx, transpose2d_kernel, grid, dim3(32, 8), 0, x, y, (int)shape[lo], (int)shape[hi], accumulate ? 1 : 0);
       talos_launched(ctx, "transpose2d");
       return TALOS_OK;
     }
@@ -266,9 +282,9 @@ TALOS_API talos_status talos_transpose(talos_ctx* ctx, const float* x, float* y,
     const unsigned run = (unsigned)(inner / vec), total = (unsigned)(n / vec), grid = (unsigned)ceil_div(total, 1024);
     const unsigned sj = run, sm = sj * (unsigned)shape[hi], si = sm * (unsigned)mid, so = si * (unsigned)shape[lo];
     const SwapArgs g{FastDiv(run), FastDiv((unsigned)shape[lo]), FastDiv((unsigned)mid), FastDiv((unsigned)shape[hi]), so, si, sm, sj};
-    if (vec == 4) swap_axes_kernel<float4><<<grid, 256, 0, ctx->stream>>>((const float4*)x, (float4*)y, total, g);
-    else if (vec == 2) swap_axes_kernel<float2><<<grid, 256, 0, ctx->stream>>>((const float2*)x, (float2*)y, total, g);
-    else swap_axes_kernel<float><<<grid, 256, 0, ctx->stream>>>(x, y, total, g);
+    if (vec == 4) talos_kernel(ctx, swap_axes_kernel<float4>, grid, 256, 0, (const float4*)x, (float4*)y, total, g);
+    else if (vec == 2) talos_kernel(ctx, swap_axes_kernel<float2>, grid, 256, 0, (const float2*)x, (float2*)y, total, g);
+    else talos_kernel(ctx, swap_axes_kernel<float>, grid, 256, 0, x, y, total, g);
     talos_launched(ctx, "transpose");
     return TALOS_OK;
   }
@@ -278,7 +294,7 @@ TALOS_API talos_status talos_transpose(talos_ctx* ctx, const float* x, float* y,
   for (int i = 0; i < rank; ++i) { a.out_shape[i] = shape[i]; a.in_stride[i] = in_stride[i]; }
   std::swap(a.out_shape[d0], a.out_shape[d1]); std::swap(a.in_stride[d0], a.in_stride[d1]);
   for (int i = rank; i < 6; ++i) { a.out_shape[i] = 1; a.in_stride[i] = 0; }
-  transpose_kernel<<<blocks_for(n), 256, 0, ctx->stream>>>(x, y, n, a, accumulate ? 1 : 0);
+  talos_kernel(ctx, transpose_kernel, blocks_for(n), 256, 0, x, y, n, a, accumulate ? 1 : 0);
   talos_launched(ctx, "transpose");
   TALOS_ENTRY_END
 }
@@ -290,12 +306,12 @@ TALOS_API talos_status talos_concat_last(talos_ctx* ctx, const float* a, const f
   int64_t n = rows * (da + db); if (n == 0) return TALOS_OK;
   TALOS_REQUIRE(a && b && out, TALOS_ERR_ARG, "null pointer");
   if (da % 4 == 0 && db % 4 == 0 && n < (1LL << 31) && aligned_to(16, a, b, out)) {
-    concat_last_vec_kernel<<<(unsigned)ceil_div(n / 4, 1024), 256, 0, ctx->stream>>>((const float4*)a, (const float4*)b, (float4*)out, (unsigned)(n / 4),
+    talos_kernel(ctx, concat_last_vec_kernel, (unsigned)ceil_div(n / 4, 1024), 256, 0, (const float4*)a, (const float4*)b, (float4*)out, (unsigned)(n / 4),
                                                                                     FastDiv((unsigned)((da + db) / 4)), (unsigned)(da / 4));
     talos_launched(ctx, "concat_last");
     return TALOS_OK;
   }
-  concat_last_kernel<<<blocks_for(n), 256, 0, ctx->stream>>>(a, b, out, rows, (int)da, (int)db);
+  talos_kernel(ctx, concat_last_kernel, blocks_for(n), 256, 0, a, b, out, rows, (int)da, (int)db);
   talos_launched(ctx, "concat_last");
   TALOS_ENTRY_END
 }
@@ -306,12 +322,12 @@ TALOS_API talos_status talos_split_last(talos_ctx* ctx, const float* g, float* g
   int64_t n = rows * (da + db); if (n == 0) return TALOS_OK;
   TALOS_REQUIRE(g, TALOS_ERR_ARG, "null pointer");
   if (da % 4 == 0 && db % 4 == 0 && n < (1LL << 31) && aligned_to(16, g, ga, gb)) {
-    split_last_vec_kernel<<<(unsigned)ceil_div(n / 4, 1024), 256, 0, ctx->stream>>>((const float4*)g, (float4*)ga, (float4*)gb, (unsigned)(n / 4),
+    talos_kernel(ctx, split_last_vec_kernel, (unsigned)ceil_div(n / 4, 1024), 256, 0, (const float4*)g, (float4*)ga, (float4*)gb, (unsigned)(n / 4),
                                                                                    FastDiv((unsigned)((da + db) / 4)), (unsigned)(da / 4), accumulate ? 1 : 0);
     talos_launched(ctx, "split_last");
     return TALOS_OK;
   }
-  split_last_kernel<<<blocks_for(n), 256, 0, ctx->stream>>>(g, ga, gb, rows, (int)da, (int)db, accumulate ? 1 : 0);
+  talos_kernel(ctx, split_last_kernel, blocks_for(n), 256, 0, g, ga, gb, rows, (int)da, (int)db, accumulate ? 1 : 0);
   talos_launched(ctx, "split_last");
   TALOS_ENTRY_END
 }
@@ -321,7 +337,7 @@ TALOS_API talos_status talos_last_token(talos_ctx* ctx, const float* x, float* y
   TALOS_REQUIRE(B >= 0 && S >= 1 && D >= 0 && D < (1 << 30), TALOS_ERR_SHAPE, "bad last_token shape");
   if (B * D == 0) return TALOS_OK;
   TALOS_REQUIRE(x && y, TALOS_ERR_ARG, "null pointer");
-  last_token_kernel<<<blocks_for(B * D), 256, 0, ctx->stream>>>(x, y, B, S, (int)D);
+  talos_kernel(ctx, last_token_kernel, blocks_for(B * D), 256, 0, x, y, B, S, (int)D);
   talos_launched(ctx, "last_token");
   TALOS_ENTRY_END
 }
@@ -331,7 +347,7 @@ TALOS_API talos_status talos_bias_add(talos_ctx* ctx, float* y, const float* bia
   TALOS_REQUIRE(rows >= 0 && n > 0 && n < (1 << 30), TALOS_ERR_SHAPE, "Add shape mismatch");
   if (rows == 0) return TALOS_OK;
   TALOS_REQUIRE(y && bias, TALOS_ERR_ARG, "null pointer");
-  bias_add_kernel<<<blocks_for(rows * n), 256, 0, ctx->stream>>>(y, bias, rows * n, (int)n);
+  talos_kernel(ctx, bias_add_kernel, blocks_for(rows * n), 256, 0, y, bias, rows * n, (int)n);
   talos_launched(ctx, "bias_add");
   TALOS_ENTRY_END
 }
@@ -342,7 +358,7 @@ TALOS_API talos_status talos_eltwise_unary(talos_ctx* ctx, int32_t op, const flo
   TALOS_REQUIRE(op >= TALOS_EW_RELU && op <= TALOS_EW_SCALE, TALOS_ERR_ARG, "bad unary op");
   TALOS_REQUIRE(n >= 0, TALOS_ERR_SHAPE, "negative length"); if (n == 0) return TALOS_OK;
   TALOS_REQUIRE(x && y, TALOS_ERR_ARG, "null pointer");
-  ew_unary_kernel<<<blocks_for(n), 256, 0, ctx->stream>>>(op, x, y, n, p0, p1);
+  talos_kernel(ctx, ew_unary_kernel, blocks_for(n), 256, 0, op, x, y, n, p0, p1);
   talos_launched(ctx, "eltwise_unary");
   TALOS_ENTRY_END
 }
@@ -352,7 +368,7 @@ TALOS_API talos_status talos_eltwise_unary_bwd(talos_ctx* ctx, int32_t op, const
   TALOS_REQUIRE(op >= TALOS_EW_RELU && op <= TALOS_EW_SCALE, TALOS_ERR_ARG, "bad unary op");
   TALOS_REQUIRE(n >= 0, TALOS_ERR_SHAPE, "negative length"); if (n == 0) return TALOS_OK;
   TALOS_REQUIRE(x && dy && dx, TALOS_ERR_ARG, "null pointer");
-  ew_unary_bwd_kernel<<<blocks_for(n), 256, 0, ctx->stream>>>(op, x, dy, dx, n, p0, p1);
+  talos_kernel(ctx, ew_unary_bwd_kernel, blocks_for(n), 256, 0, op, x, dy, dx, n, p0, p1);
   talos_launched(ctx, "eltwise_unary_bwd");
   TALOS_ENTRY_END
 }
@@ -364,9 +380,9 @@ TALOS_API talos_status talos_eltwise_binary(talos_ctx* ctx, int32_t op, const fl
   TALOS_REQUIRE(a && b && y, TALOS_ERR_ARG, "null pointer");
   if (aligned_to(16, a, b, y)) {
     const int64_t n4 = n / 4; const int rest = (int)(n & 3);
-    ew_binary_kernel<float4><<<(unsigned)(ceil_div(n4, 512) + (rest ? 1 : 0)), 256, 0, ctx->stream>>>(op, (const float4*)a, (const float4*)b, (float4*)y, n4, rest);
+    talos_kernel(ctx, ew_binary_kernel<float4>, (unsigned)(ceil_div(n4, 512) + (rest ? 1 : 0)), 256, 0, op, (const float4*)a, (const float4*)b, (float4*)y, n4, rest);
   } else {
-    ew_binary_kernel<float><<<(unsigned)ceil_div(n, 512), 256, 0, ctx->stream>>>(op, a, b, y, n, 0);
+    talos_kernel(ctx, ew_binary_kernel<float>, (unsigned)ceil_div(n, 512), 256, 0, op, a, b, y, n, 0);
   }
   talos_launched(ctx, "eltwise_binary");
   TALOS_ENTRY_END
@@ -377,7 +393,7 @@ TALOS_API talos_status talos_eltwise_binary_bwd(talos_ctx* ctx, int32_t op, cons
   TALOS_REQUIRE(op >= TALOS_EW_ADD && op <= TALOS_EW_DIV, TALOS_ERR_ARG, "bad binary op");
   TALOS_REQUIRE(n >= 0, TALOS_ERR_SHAPE, "negative length"); if (n == 0) return TALOS_OK;
   TALOS_REQUIRE(a && b && dy, TALOS_ERR_ARG, "null pointer");
-  ew_binary_bwd_kernel<<<blocks_for(n), 256, 0, ctx->stream>>>(op, a, b, dy, da, db, n);
+  talos_kernel(ctx, ew_binary_bwd_kernel, blocks_for(n), 256, 0, op, a, b, dy, da, db, n);
   talos_launched(ctx, "eltwise_binary_bwd");
   TALOS_ENTRY_END
 }
@@ -388,9 +404,9 @@ TALOS_API talos_status talos_reduce_sum(talos_ctx* ctx, const float* x, int64_t 
   TALOS_REQUIRE(out && (x || n == 0), TALOS_ERR_ARG, "null pointer");
   int parts = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 1024), 1024));
   float* partial = (float*)talos_workspace(ctx, sizeof(float) * parts);
-  reduce_stage1_kernel<<<parts, 256, 0, ctx->stream>>>(x, n, partial);
+  talos_kernel(ctx, reduce_stage1_kernel, parts, 256, 0, x, n, partial);
   talos_launched(ctx, "reduce_stage1");
-  reduce_stage2_kernel<<<1, 256, 0, ctx->stream>>>(partial, parts, scale, out, accumulate ? 1 : 0);
+  talos_kernel(ctx, reduce_stage2_kernel, 1, 256, 0, partial, parts, scale, out, accumulate ? 1 : 0);
   talos_launched(ctx, "reduce_stage2");
   TALOS_ENTRY_END
 }
@@ -399,7 +415,7 @@ TALOS_API talos_status talos_fill_from_scalar(talos_ctx* ctx, const float* s, fl
   talos_check_ctx(ctx);
   TALOS_REQUIRE(n >= 0, TALOS_ERR_SHAPE, "negative length"); if (n == 0) return TALOS_OK;
   TALOS_REQUIRE(s && y, TALOS_ERR_ARG, "null pointer");
-  fill_from_scalar_kernel<<<blocks_for(n), 256, 0, ctx->stream>>>(s, scale, y, n, accumulate ? 1 : 0);
+  talos_kernel(ctx, fill_from_scalar_kernel, blocks_for(n), 256, 0, s, scale, y, n, accumulate ? 1 : 0);
   talos_launched(ctx, "fill_from_scalar");
   TALOS_ENTRY_END
 }

@@ -35,6 +35,7 @@ constexpr unsigned XCHG_DEFAULT_SPINS = 1u << 22;
 
 __global__ void __launch_bounds__(256)
 xchg_adam_kernel(XchgAdamArgs a) {
+  talos_pdl();
   __shared__ int sh_ok;
   __shared__ float sh_count;
   if (threadIdx.x == 0) {
@@ -105,6 +106,6 @@ void talos_xchg_adam_launch(talos_ctx* ctx, const XchgAdamArgs& a_in) {
   XchgAdamArgs a = a_in;
   if (a.spins == 0) a.spins = XCHG_DEFAULT_SPINS;
   const long long groups = (a.n >> 2) + 1;             // + the tail group
-  xchg_adam_kernel<<<(unsigned)ceil_div(groups, 256), 256, 0, ctx->stream>>>(a);
+  talos_kernel(ctx, xchg_adam_kernel, (unsigned)ceil_div(groups, 256), 256, 0, a);
   talos_launched(ctx, "xchg_adam");
 }

@@ -54,6 +54,7 @@ __device__ __forceinline__ void gae_load(const GaeArgs& g, long long t0, bool al
 template <int PASS>
 __global__ void __launch_bounds__(GAE_THREADS)
 gae_scan_kernel(GaeArgs g, int aligned, Affine* block_maps, const float* __restrict__ carries, float* __restrict__ advantages, float* __restrict__ returns) {
+  talos_pdl(block_maps, carries, advantages, returns);
   __shared__ Affine warp_maps[GAE_THREADS / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long long t0 = (long long)blockIdx.x * GAE_CHUNK + (long long)tid * GAE_PER_THREAD;
@@ -105,6 +106,7 @@ gae_scan_kernel(GaeArgs g, int aligned, Affine* block_maps, const float* __restr
 constexpr int CHAIN_THREADS = 1024;
 __global__ void __launch_bounds__(CHAIN_THREADS)
 gae_chain_kernel(const Affine* __restrict__ block_maps, float* __restrict__ carries, int blocks) {
+  talos_pdl(block_maps, carries);
   __shared__ Affine sh[CHAIN_THREADS];
   const int tid = threadIdx.x, per = (blocks + CHAIN_THREADS - 1) / CHAIN_THREADS;
   const int b0 = tid * per, b1 = min(blocks, b0 + per);
@@ -138,6 +140,7 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
 template <int SQDIFF>
 __global__ void __launch_bounds__(RED_THREADS)
 moment_partial_kernel(const float* __restrict__ x, long long n, int vec, const float* __restrict__ stats, double* __restrict__ partials) {
+  talos_pdl(x, stats, partials);
   __shared__ double sh[RED_THREADS / 32];
   const float mean = SQDIFF ? stats[0] : 0.f;
   const long long stride = (long long)gridDim.x * RED_THREADS, first = (long long)blockIdx.x * RED_THREADS + threadIdx.x;
@@ -158,6 +161,7 @@ moment_partial_kernel(const float* __restrict__ x, long long n, int vec, const f
 template <int SQDIFF>
 __global__ void __launch_bounds__(RED_THREADS)
 moment_final_kernel(const double* __restrict__ partials, int count, long long n, float* stats) {
+  talos_pdl(partials, stats);
   __shared__ double sh[RED_THREADS];
   double acc = 0.0;
   for (int i = threadIdx.x; i < count; i += RED_THREADS) acc += partials[i];
@@ -169,6 +173,7 @@ moment_final_kernel(const double* __restrict__ partials, int count, long long n,
   if (SQDIFF) stats[1] = (float)(sqrt(s / (double)n) + 1e-8); else stats[0] = (float)(s / (double)n);
 }
 __global__ void normalize_kernel(const float* x, long long n, int vec, const float* __restrict__ stats, float* y) {
+  talos_pdl(x, stats, y);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const float mean = stats[0], sd = stats[1];
   if (vec) {
@@ -199,11 +204,11 @@ TALOS_API talos_status talos_gae(talos_ctx* ctx, const float* rewards, const flo
   Affine* maps = (Affine*)ws; float* carries = (float*)(maps + blocks);
   GaeArgs g{rewards, values, terminals, len, gamma, gamma * lambda, rew_mean, (float)(1.0 / (std::sqrt((double)rew_var) + 1e-8))};
   const int aligned = ((((uintptr_t)rewards | (uintptr_t)values | (uintptr_t)terminals | (uintptr_t)advantages | (uintptr_t)returns) & 15) == 0) ? 1 : 0;
-  gae_scan_kernel<0><<<blocks, GAE_THREADS, 0, ctx->stream>>>(g, aligned, maps, nullptr, nullptr, nullptr);
+  talos_kernel(ctx, gae_scan_kernel<0>, blocks, GAE_THREADS, 0, g, aligned, maps, nullptr, nullptr, nullptr);
   talos_launched(ctx, "gae_scan (fold)");
-  gae_chain_kernel<<<1, CHAIN_THREADS, 0, ctx->stream>>>(maps, carries, blocks);
+  talos_kernel(ctx, gae_chain_kernel, 1, CHAIN_THREADS, 0, maps, carries, blocks);
   talos_launched(ctx, "gae_chain");
-  gae_scan_kernel<1><<<blocks, GAE_THREADS, 0, ctx->stream>>>(g, aligned, maps, carries, advantages, returns);
+  talos_kernel(ctx, gae_scan_kernel<1>, blocks, GAE_THREADS, 0, g, aligned, maps, carries, advantages, returns);
   talos_launched(ctx, "gae_scan (replay)");
   TALOS_ENTRY_END
 }
@@ -219,15 +224,15 @@ TALOS_API talos_status talos_normalize_slice(talos_ctx* ctx, const float* x, int
   char* ws = (char*)talos_workspace(ctx, sizeof(double) * (size_t)blocks + 16);
   double* partials = (double*)ws;
   float* st = stats ? stats : (float*)(partials + blocks);
-  moment_partial_kernel<0><<<blocks, RED_THREADS, 0, ctx->stream>>>(x, n, vec, st, partials);
+  talos_kernel(ctx, moment_partial_kernel<0>, blocks, RED_THREADS, 0, x, n, vec, st, partials);
   talos_launched(ctx, "moment_partial (sum)");
-  moment_final_kernel<0><<<1, RED_THREADS, 0, ctx->stream>>>(partials, blocks, n, st);
+  talos_kernel(ctx, moment_final_kernel<0>, 1, RED_THREADS, 0, partials, blocks, n, st);
   talos_launched(ctx, "moment_final (mean)");
-  moment_partial_kernel<1><<<blocks, RED_THREADS, 0, ctx->stream>>>(x, n, vec, st, partials);
+  talos_kernel(ctx, moment_partial_kernel<1>, blocks, RED_THREADS, 0, x, n, vec, st, partials);
   talos_launched(ctx, "moment_partial (squared differences)");
-  moment_final_kernel<1><<<1, RED_THREADS, 0, ctx->stream>>>(partials, blocks, n, st);
+  talos_kernel(ctx, moment_final_kernel<1>, 1, RED_THREADS, 0, partials, blocks, n, st);
   talos_launched(ctx, "moment_final (std)");
-  normalize_kernel<<<(unsigned)ceil_div(vec ? ceil_div(n, 4) : n, 256), 256, 0, ctx->stream>>>(x, n, vec, st, y);
+  talos_kernel(ctx, normalize_kernel, (unsigned)ceil_div(vec ? ceil_div(n, 4) : n, 256), 256, 0, x, n, vec, st, y);
   talos_launched(ctx, "normalize");
   TALOS_ENTRY_END
 }

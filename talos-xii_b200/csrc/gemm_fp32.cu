@@ -22,6 +22,7 @@ struct GemmArgs {
 template <int BM, int BN, int BK, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 gemm_fp32_kernel(GemmArgs g) {
+  talos_pdl();
   constexpr int NT = (BM / TM) * (BN / TN);
   __shared__ float As[2][BK][BM + 4];
   __shared__ float Bs[2][BK][BN + 4];
@@ -55,14 +56,14 @@ gemm_fp32_kernel(GemmArgs g) {
       int e = tid + i * NT, m, k;
       if (a_k_contig) { k = e % BK; m = e / BK; } else { m = e % BM; k = e / BM; }
       int gm = m0 + m, gk = k0 + k;
-      ra[i] = (gm < g.M && gk < k_end) ? __ldg(A + (long long)gm * g.sAm + (long long)gk * g.sAk) : 0.f;
+      ra[i] = (gm < g.M && gk < k_end) ? A[(long long)gm * g.sAm + (long long)gk * g.sAk] : 0.f;
     }
 #pragma unroll
     for (int i = 0; i < B_ELEMS; ++i) {
       int e = tid + i * NT, n, k;
       if (b_n_contig) { n = e % BN; k = e / BN; } else { k = e % BK; n = e / BK; }
       int gn = n0 + n, gk = k0 + k;
-      rb[i] = (gn < g.N && gk < k_end) ? __ldg(B + (long long)gk * g.sBk + (long long)gn * g.sBn) : 0.f;
+      rb[i] = (gn < g.N && gk < k_end) ? B[(long long)gk * g.sBk + (long long)gn * g.sBn] : 0.f;
     }
   };
   auto store_tiles = [&](int buf) {
@@ -131,6 +132,7 @@ gemm_fp32_kernel(GemmArgs g) {
 // epilogue.  Scalar version for ragged shapes.
 __global__ void talos_splitk_reduce_kernel(const float* __restrict__ partial, int splits, long long M, long long N,
                                            float* C, long long ldc, EpiArgs epi) {
+  talos_pdl(partial, C);
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= M * N) return;
   long long m = idx / N, n = idx % N;
@@ -145,6 +147,7 @@ __global__ void talos_splitk_reduce_kernel(const float* __restrict__ partial, in
 __global__ void __launch_bounds__(256)
 talos_splitk_reduce_vec_kernel(const float4* __restrict__ partial, int splits, long long MN4, long long N, float* C,
                                long long ldc, EpiArgs epi) {
+  talos_pdl(partial, C);
   __shared__ float4 sh[4][64];
   const int col = threadIdx.x & 63, sl = threadIdx.x >> 6;
   const long long idx = (long long)blockIdx.x * 64 + col;
@@ -172,9 +175,9 @@ void talos_splitk_reduce(talos_ctx* ctx, const float* partial, int splits, int64
                          int64_t ldc, const EpiArgs& epi) {
   int64_t total = M * N;
   if ((N & 3) == 0 && (((uintptr_t)partial) & 15) == 0) {
-    talos_splitk_reduce_vec_kernel<<<(unsigned)ceil_div(total / 4, 64), 256, 0, ctx->stream>>>((const float4*)partial, splits, total / 4, N, C, ldc, epi);
+    talos_kernel(ctx, talos_splitk_reduce_vec_kernel, (unsigned)ceil_div(total / 4, 64), 256, 0, (const float4*)partial, splits, total / 4, N, C, ldc, epi);
   } else {
-    talos_splitk_reduce_kernel<<<(unsigned)ceil_div(total, 256), 256, 0, ctx->stream>>>(partial, splits, M, N, C, ldc, epi);
+    talos_kernel(ctx, talos_splitk_reduce_kernel, (unsigned)ceil_div(total, 256), 256, 0, partial, splits, M, N, C, ldc, epi);
   }
   talos_launched(ctx, "splitk_reduce");
 }
@@ -208,7 +211,7 @@ void talos_gemm_fp32_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t
     g.partial = (float*)talos_workspace(ctx, sizeof(float) * (size_t)splits * M * N);
   }
   dim3 grid((unsigned)ceil_div(N, 128), (unsigned)ceil_div(M, 128), (unsigned)(splits > 1 ? splits : batch));
-  gemm_fp32_kernel<128, 128, 16, 8, 8><<<grid, 256, 0, ctx->stream>>>(g);
+  talos_kernel(ctx, gemm_fp32_kernel<128, 128, 16, 8, 8>, grid, 256, 0, g);
   talos_launched(ctx, "gemm_fp32");
   if (splits > 1) talos_splitk_reduce(ctx, g.partial, splits, M, N, C, ldc, epi);
 }

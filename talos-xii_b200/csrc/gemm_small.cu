@@ -245,6 +245,7 @@ __device__ __forceinline__ void small_product(const SmallProduct& g, unsigned it
 template <int BM, int BN, int TM, int KG, int KC, bool VEC>
 __global__ void __launch_bounds__((SmallCfg<BM, BN, TM, KG, KC>::T), (BM <= 32 ? 2 : 1))
 gemm_small_kernel(const __grid_constant__ SmallProduct g) {
+  talos_pdl();
   extern __shared__ __align__(16) float sm[];
   small_product<BM, BN, TM, KG, KC, VEC, false>(g, blockIdx.x, sm);
 }
@@ -254,6 +255,7 @@ gemm_small_kernel(const __grid_constant__ SmallProduct g) {
 template <int BM, int BN, int TM, int KG, int KC, bool VEC>
 __global__ void __launch_bounds__((SmallCfg<BM, BN, TM, KG, KC>::T), (BM <= 32 ? 2 : 1))
 linear_bwd_small_kernel(const __grid_constant__ SmallProduct gx, const __grid_constant__ SmallProduct gw, unsigned items_w) {
+  talos_pdl();
   extern __shared__ __align__(16) float sm[];
   const bool w_role = blockIdx.x < items_w;
   small_product<BM, BN, TM, KG, KC, VEC, true>(w_role ? gw : gx, w_role ? blockIdx.x : blockIdx.x - items_w, sm);
@@ -272,23 +274,13 @@ void small_shape(talos_ctx* ctx, SmallProduct& g, int bm, int kc, int64_t batch,
   g.splits = splits; g.k_split = (int)(ceil_div(chunks, splits) * kc);
 }
 int small_tile(talos_ctx* ctx, int64_t tiles16, int64_t tiles32) { return tiles16 <= 2 * ctx->sm_count ? 16 : tiles32 <= 2 * ctx->sm_count ? 32 : 64; }
-template <typename... Params, typename... Args>
-void small_launch(talos_ctx* ctx, void (*kern)(Params...), int64_t items, int cluster, int threads, size_t smem, Args... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(ceil_div(items, cluster) * cluster)); cfg.blockDim = dim3((unsigned)threads); cfg.dynamicSmemBytes = smem; cfg.stream = ctx->stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = cluster > 1 ? 1 : 0;
-  TALOS_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
-}
 template <int BM, int TM, int KG, int KC, bool VEC>
 void launch_gemm(talos_ctx* ctx, SmallProduct& g, int64_t batch, int64_t slots) {
   using Cfg = SmallCfg<BM, BM, TM, KG, KC>;
   small_shape(ctx, g, BM, KC, batch, slots);
   static std::atomic<uint64_t> smem_set{0};
   talos_allow_smem(smem_set, (const void*)gemm_small_kernel<BM, BM, TM, KG, KC, VEC>, Cfg::BYTES, ctx->device);
-  small_launch(ctx, gemm_small_kernel<BM, BM, TM, KG, KC, VEC>, (int64_t)g.m_tiles * g.n_tiles * batch * g.splits, g.splits, Cfg::T, Cfg::BYTES, g);
+  talos_kernel_cluster(ctx, gemm_small_kernel<BM, BM, TM, KG, KC, VEC>, (unsigned)((int64_t)g.m_tiles * g.n_tiles * batch * g.splits), Cfg::T, Cfg::BYTES, g.splits, g);
 }
 template <int BM, int TM, int KG, int KC, bool VEC>
 void launch_bwd(talos_ctx* ctx, SmallProduct& gx, SmallProduct& gw, int64_t slots) {
@@ -304,7 +296,8 @@ void launch_bwd(talos_ctx* ctx, SmallProduct& gx, SmallProduct& gw, int64_t slot
   items_w = ceil_div(items_w, cluster) * cluster;
   static std::atomic<uint64_t> smem_set{0};
   talos_allow_smem(smem_set, (const void*)linear_bwd_small_kernel<BM, BM, TM, KG, KC, VEC>, Cfg::BYTES, ctx->device);
-  small_launch(ctx, linear_bwd_small_kernel<BM, BM, TM, KG, KC, VEC>, items_w + items_x, cluster, Cfg::T, Cfg::BYTES, gx, gw, (unsigned)items_w);
+  talos_kernel_cluster(ctx, linear_bwd_small_kernel<BM, BM, TM, KG, KC, VEC>, (unsigned)(items_w + ceil_div(items_x, cluster) * cluster), Cfg::T, Cfg::BYTES, cluster, gx, gw,
+                       (unsigned)items_w);
 }
 
 }  // namespace

@@ -91,6 +91,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tmap_a, const CU
   }
   if (warp == 1) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
   tc_fence_before();
+  talos_pdl();                             // barriers and tensor memory were set up beside the previous kernel's tail; from here on memory is read
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
@@ -363,6 +364,7 @@ gemm_tc_aux_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
 // mode the tensor core TRUNCATES its fp32 inputs, a bias of ~3.5e-4 per operand; pre-rounding the small operand
 // (the weights) removes its half of that bias for a few microseconds of extra work.
 __global__ void round_tf32_kernel(const float* __restrict__ in, long long ld, int rows, int cols, int out_ld, float* __restrict__ out) {
+  talos_pdl(in, out);
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)rows * out_ld) return;
   int r = (int)(idx / out_ld), c = (int)(idx % out_ld);
@@ -372,6 +374,7 @@ __global__ void round_tf32_kernel(const float* __restrict__ in, long long ld, in
 // Dense TF32 hi / lo copies of a [rows][cols] matrix: hi = rna(a), lo = rna(a - hi).
 __global__ void split_tf32_kernel(const float* __restrict__ in, long long ld, int rows, int cols, int out_ld, float* __restrict__ hi,
                                   float* __restrict__ lo) {
+  talos_pdl(in, hi, lo);
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)rows * out_ld) return;
   int r = (int)(idx / out_ld), c = (int)(idx % out_ld);
@@ -472,7 +475,7 @@ void launch_one(talos_ctx* ctx, const CUtensorMap& ta, const CUtensorMap& tb, co
   size_t smem = tc_smem_bytes<BN, STAGES, X3, SBUF, EW>();
   static std::atomic<uint64_t> smem_set{0};
   talos_allow_smem(smem_set, (const void*)kern, smem, ctx->device);
-  kern<<<grid, TcRoles<X3, BPS, BN, EW>::THREADS, smem, ctx->stream>>>(ta, tb, tc, tbl, g);
+  talos_kernel(ctx, kern, grid, TcRoles<X3, BPS, BN, EW>::THREADS, smem, ta, tb, tc, tbl, g);
   talos_launched(ctx, "gemm_tcgen05");
 }
 
@@ -609,13 +612,13 @@ void tc_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K
     B = extra->b_hi; B_lo = x3 ? extra->b_lo : nullptr;
   } else if (presplit) {
     float* hi = (float*)(scratch + partial_bytes); float* lo = hi + b_rows * s_ld;
-    split_tf32_kernel<<<(unsigned)ceil_div(b_rows * s_ld, 256), 256, 0, ctx->stream>>>(B, ldb, (int)b_rows, (int)b_cols, (int)s_ld, hi, lo);
+    talos_kernel(ctx, split_tf32_kernel, (unsigned)ceil_div(b_rows * s_ld, 256), 256, 0, B, ldb, (int)b_rows, (int)b_cols, (int)s_ld, hi, lo);
     talos_launched(ctx, "split_tf32");
     B = hi; B_lo = lo; ldb = s_ld;
   }
   if (round_a || round_b) {
     float* dst = (float*)(scratch + partial_bytes);
-    round_tf32_kernel<<<(unsigned)ceil_div(r_rows * r_ld, 256), 256, 0, ctx->stream>>>(round_a ? A : B, round_a ? lda : ldb, (int)r_rows, (int)r_cols, (int)r_ld, dst);
+    talos_kernel(ctx, round_tf32_kernel, (unsigned)ceil_div(r_rows * r_ld, 256), 256, 0, round_a ? A : B, round_a ? lda : ldb, (int)r_rows, (int)r_cols, (int)r_ld, dst);
     talos_launched(ctx, "round_tf32");
     if (round_a) { A = dst; lda = r_ld; } else { B = dst; ldb = r_ld; }
   }
@@ -656,7 +659,7 @@ void tc_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K
   { const size_t smem = tc_smem_bytes<BNv, ST, X3v, SB, EWv>() + 128;                                                               \
     static std::atomic<uint64_t> smem_set{0};                                                                                       \
     talos_allow_smem(smem_set, (const void*)gemm_tc_aux_kernel<BNv, ST, X3v, SB, EWv>, smem, ctx->device);                          \
-    gemm_tc_aux_kernel<BNv, ST, X3v, SB, EWv><<<grid, TcRoles<X3v, X3v, BNv, EWv>::THREADS, smem, ctx->stream>>>(ta, tb, tc, tbl, tx, g); }
+    talos_kernel(ctx, gemm_tc_aux_kernel<BNv, ST, X3v, SB, EWv>, grid, TcRoles<X3v, X3v, BNv, EWv>::THREADS, smem, ta, tb, tc, tbl, tx, g); }
     if (!x3) TALOS_TC_AUX(256, 3, false, 2, 0)
     else if (bn == 128 && wide_epi) TALOS_TC_AUX(128, 2, true, 1, 16)
     else if (bn == 128) TALOS_TC_AUX(128, 2, true, 2, 0)

@@ -89,6 +89,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   }
   if (warp == 1) { tmem_alloc2(tmem_slot, TMEM_COLS); tmem_relinquish2(); }
   tc_fence_before();
+  talos_pdl();
   __syncthreads();
   cluster_sync();                                              // the peer's barriers exist before anything is signalled on them
   tc_fence_after();
@@ -257,7 +258,7 @@ void launch2_one(talos_ctx* ctx, const CUtensorMap& ta, const CUtensorMap& tb, c
   size_t smem = tc2_smem_bytes<BN, STAGES, X3>();
   static std::atomic<uint64_t> smem_set{0};
   talos_allow_smem(smem_set, (const void*)kern, smem, ctx->device);
-  kern<<<grid, X3 ? 448 : 320, smem, ctx->stream>>>(ta, tb, tc, tbl, g);
+  talos_kernel(ctx, kern, grid, X3 ? 448 : 320, smem, ta, tb, tc, tbl, g);
   talos_launched(ctx, "gemm_tcgen05_2cta");
 }
 template <int BN, int STAGES, bool X3, bool BPS>

@@ -4,6 +4,7 @@
 namespace {
 __global__ void dact_mul_kernel(const float* __restrict__ dy, const float* __restrict__ saved, float* __restrict__ dz,
                                 long long n, int act) {
+  talos_pdl(dy, saved, dz);
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dz[i] = dy[i] * talos_dact(saved[i], act);
 }
@@ -12,6 +13,7 @@ __global__ void dact_mul_kernel(const float* __restrict__ dy, const float* __res
 template <int ACT>
 __global__ void __launch_bounds__(256)
 dact_mul_vec_kernel(const float4* __restrict__ dy, const float4* __restrict__ saved, float4* __restrict__ dz, long long n4) {
+  talos_pdl(dy, saved, dz);
   const long long i = (long long)blockIdx.x * 512 + threadIdx.x;
   float4 g[2], s[2];
 #pragma unroll
@@ -24,9 +26,9 @@ dact_mul_vec_kernel(const float4* __restrict__ dy, const float4* __restrict__ sa
 void dact_mul(talos_ctx* ctx, const float* dy, const float* saved, float* dz, int64_t n, int act) {
   if (n % 4 == 0 && (((uintptr_t)dy | (uintptr_t)saved | (uintptr_t)dz) & 15) == 0) {
     auto kern = act == TALOS_ACT_RELU ? dact_mul_vec_kernel<TALOS_ACT_RELU> : act == TALOS_ACT_TANH ? dact_mul_vec_kernel<TALOS_ACT_TANH> : dact_mul_vec_kernel<TALOS_ACT_SILU>;
-    kern<<<(unsigned)ceil_div(n / 4, 512), 256, 0, ctx->stream>>>((const float4*)dy, (const float4*)saved, (float4*)dz, n / 4);
+    talos_kernel(ctx, kern, (unsigned)ceil_div(n / 4, 512), 256, 0, (const float4*)dy, (const float4*)saved, (float4*)dz, n / 4);
   } else {
-    dact_mul_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, ctx->stream>>>(dy, saved, dz, n, act);
+    talos_kernel(ctx, dact_mul_kernel, (unsigned)ceil_div(n, 256), 256, 0, dy, saved, dz, n, act);
   }
   talos_launched(ctx, "dact_mul");
 }

@@ -16,6 +16,7 @@ ppo_loss_kernel(const float* __restrict__ logits, long long ld, const float* __r
                 const float* __restrict__ ret, long long n, int n_actions, float clip, float c_v, float c_h, float inv_denom,
                 float* __restrict__ dlogits, long long ld_out, float* __restrict__ dvalues, long long dvs,
                 float* __restrict__ partial, int vec, int32_t* __restrict__ status, float* __restrict__ colsum_part, int cs_width) {
+  talos_pdl(logits, values, actions, old_logp, adv, ret, dlogits, dvalues, partial, status, colsum_part);
   __shared__ float sh_loss[128], sh_kl[128];
   __shared__ float sh_cs[4][MAX_ACTIONS + 1];
   const bool want_cs = colsum_part != nullptr;                 // block-uniform
@@ -127,6 +128,7 @@ ppo_loss_kernel(const float* __restrict__ logits, long long ld, const float* __r
 
 // Sums the per-block (loss, kl) partials in block order and adds {loss, kl, n} to stats.
 __global__ void ppo_stats_kernel(const float* __restrict__ partial, int nblocks, float n, float* stats) {
+  talos_pdl(partial, stats);
   __shared__ float sl[256], sk[256];
   float a = 0.f, b = 0.f;
   for (int i = threadIdx.x; i < nblocks; i += 256) { a += partial[2 * i]; b += partial[2 * i + 1]; }
@@ -136,6 +138,7 @@ __global__ void ppo_stats_kernel(const float* __restrict__ partial, int nblocks,
 }
 
 __global__ void sumsq_stage1_kernel(const float* __restrict__ g, long long n, float scale, float* __restrict__ partial) {
+  talos_pdl(g, partial);
   __shared__ float sh[256];
   float s = 0.f;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) { float v = g[i] * scale; s += v * v; }
@@ -150,6 +153,7 @@ __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, 
                             long long n, float lr, float b1, float b2, float eps, float inv_bc1, float inv_bc2,
                             float grad_scale, const float* __restrict__ norm_partial, int nparts, float clip_norm,
                             const float* __restrict__ count_ptr, float* __restrict__ stats_out) {
+  talos_pdl(p, g, m, v, norm_partial, count_ptr, stats_out);
   float coef = grad_scale;
   if (count_ptr) {                       // gradients hold sums over `count` samples (the tail of the flat buffer)
     coef = grad_scale / fmaxf(count_ptr[0], 1.f);
@@ -180,7 +184,7 @@ int talos_ppo_loss_launch(talos_ctx* ctx, const float* logits, int64_t ld_logits
                           float c_entropy, float denom, float* dlogits, int64_t ld_out, float* dvalues, int64_t dvalue_stride, float* partial,
                           float* colsum_part, int cs_width) {
   const int blocks = (int)ceil_div(n, 128);
-#define TALOS_PPO_LAUNCH(A) ppo_loss_kernel<A><<<blocks, 128, 0, ctx->stream>>>(logits, ld_logits, values, value_stride, actions, old_logp, adv, ret, n, n_actions, clip, c_value, c_entropy, 1.f / denom, dlogits, ld_out, dvalues, dvalue_stride, partial, vec, ctx->dev_status, colsum_part, cs_width)
+#define TALOS_PPO_LAUNCH(A) talos_kernel(ctx, ppo_loss_kernel<A>, blocks, 128, 0, logits, ld_logits, values, value_stride, actions, old_logp, adv, ret, n, n_actions, clip, c_value, c_entropy, 1.f / denom, dlogits, ld_out, dvalues, dvalue_stride, partial, vec, ctx->dev_status, colsum_part, cs_width)
   const int vec = (((uintptr_t)logits | (uintptr_t)dlogits) & 15) == 0 && ld_logits % 4 == 0 && ld_out % 4 == 0;
   if (n_actions == 16) TALOS_PPO_LAUNCH(16); else if (n_actions == 5) TALOS_PPO_LAUNCH(5); else TALOS_PPO_LAUNCH(0);
 #undef TALOS_PPO_LAUNCH
@@ -204,7 +208,7 @@ TALOS_API talos_status talos_ppo_loss_fwd_bwd(talos_ctx* ctx, const float* logit
   float* partial = (float*)talos_workspace(ctx, sizeof(float) * 2 * (size_t)blocks);
   talos_ppo_loss_launch(ctx, logits, ld_logits, values, value_stride, actions, old_logp, adv, ret, n, n_actions, clip, c_value, c_entropy, denom, dlogits,
                         ld_out, dvalues, dvalue_stride, partial, nullptr, 0);
-  ppo_stats_kernel<<<1, 256, 0, ctx->stream>>>(partial, blocks, (float)n, stats);
+  talos_kernel(ctx, ppo_stats_kernel, 1, 256, 0, partial, blocks, (float)n, stats);
   talos_launched(ctx, "ppo_stats");
   TALOS_ENTRY_END
 }
@@ -217,10 +221,10 @@ void talos_adam_launch(talos_ctx* ctx, float* params, const float* grads, float*
   if (clip_norm > 0.f) {
     nparts = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 4096), 64));
     norm_partial = (float*)talos_workspace(ctx, sizeof(float) * nparts);
-    sumsq_stage1_kernel<<<nparts, 256, 0, ctx->stream>>>(grads, n, grad_scale, norm_partial);
+    talos_kernel(ctx, sumsq_stage1_kernel, nparts, 256, 0, grads, n, grad_scale, norm_partial);
     talos_launched(ctx, "adam_sumsq");
   }
-  adam_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, ctx->stream>>>(params, grads, m, v, n, lr, beta1, beta2, eps, (float)(1.0 / bc1),
+  talos_kernel(ctx, adam_kernel, (unsigned)ceil_div(n, 256), 256, 0, params, grads, m, v, n, lr, beta1, beta2, eps, (float)(1.0 / bc1),
                                                                   (float)(1.0 / bc2), grad_scale, norm_partial, nparts, clip_norm,
                                                                   count_ptr, stats_out);
   talos_launched(ctx, "adam");
@@ -235,7 +239,7 @@ TALOS_API talos_status talos_adam_step_global_clip(talos_ctx* ctx, float* params
   if (n == 0) return TALOS_OK;
   TALOS_REQUIRE(params && grads && m && v && sumsq_dev, TALOS_ERR_ARG, "null pointer");
   const double bc1 = 1.0 - pow((double)beta1, (double)t), bc2 = 1.0 - pow((double)beta2, (double)t);
-  adam_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, ctx->stream>>>(params, grads, m, v, n, lr, beta1, beta2, eps, (float)(1.0 / bc1), (float)(1.0 / bc2),
+  talos_kernel(ctx, adam_kernel, (unsigned)ceil_div(n, 256), 256, 0, params, grads, m, v, n, lr, beta1, beta2, eps, (float)(1.0 / bc1), (float)(1.0 / bc2),
                                                                   grad_scale, sumsq_dev, 1, clip_norm, nullptr, nullptr);
   talos_launched(ctx, "adam_global_clip");
   TALOS_ENTRY_END

@@ -61,6 +61,7 @@ int gemm_dw(talos_ppo* p, int64_t M, int64_t N, int64_t K, const float* A, int64
 }
 
 __global__ void prepare_weights_kernel(const float* __restrict__ w, float* __restrict__ hi, float* __restrict__ lo, long long n) {
+  talos_pdl(w, hi, lo);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float a = w[i];
@@ -70,7 +71,7 @@ __global__ void prepare_weights_kernel(const float* __restrict__ w, float* __res
 }
 void ensure_weights_prepared(talos_ppo* p) {
   if (!p->w_hi || p->weights_prepared) return;
-  prepare_weights_kernel<<<(unsigned)ceil_div(p->n_int, 256), 256, 0, p->ctx->stream>>>(p->params, p->w_hi, p->w_lo, p->n_int);
+  talos_kernel(p->ctx, prepare_weights_kernel, (unsigned)ceil_div(p->n_int, 256), 256, 0, p->params, p->w_hi, p->w_lo, p->n_int);
   talos_launched(p->ctx, "prepare_weights");
   p->weights_prepared = true;
 }
@@ -83,6 +84,7 @@ constexpr int GRAD_SEGS = 7;
 struct GradSegs { float* dst[GRAD_SEGS]; const float* src[GRAD_SEGS]; int n[GRAD_SEGS]; int slabs[GRAD_SEGS]; int first_block[GRAD_SEGS + 1]; float count; };
 __global__ void __launch_bounds__(256)
 grad_gather_kernel(GradSegs g) {
+  talos_pdl();
   __shared__ float sh[8][33];
   int s = 0;
   while (s < GRAD_SEGS - 1 && (int)blockIdx.x >= g.first_block[s + 1]) ++s;
@@ -107,6 +109,7 @@ grad_gather_kernel(GradSegs g) {
 }
 
 __global__ void unpack_heads_kernel(const float* __restrict__ z, int HP, int A, long long n, float* __restrict__ logits, float* __restrict__ values) {
+  talos_pdl(z, logits, values);
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n * (A + 1)) return;
   long long r = i / (A + 1); int c = (int)(i % (A + 1));
@@ -115,6 +118,7 @@ __global__ void unpack_heads_kernel(const float* __restrict__ z, int HP, int A, 
 }
 __global__ void log_prob_kernel(const float* __restrict__ z, int HP, int A, const int* __restrict__ actions, long long n, float* __restrict__ out,
                                 int32_t* __restrict__ status) {
+  talos_pdl(z, actions, out, status);
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float* l = z + i * HP; float mx = -INFINITY;
@@ -255,7 +259,7 @@ void step(talos_ppo* p, talos_comm* comm, const float* obs, const int32_t* actio
     int blocks = 0;
     for (int i = 0; i < GRAD_SEGS; ++i) { gs.first_block[i] = blocks; if (gs.slabs[i] > 0) blocks += (int)ceil_div(gs.n[i], 32); }
     gs.first_block[GRAD_SEGS] = blocks;
-    if (blocks > 0) { grad_gather_kernel<<<blocks, 256, 0, ctx->stream>>>(gs); talos_launched(ctx, "grad_gather"); }
+    if (blocks > 0) { talos_kernel(ctx, grad_gather_kernel, blocks, 256, 0, gs); talos_launched(ctx, "grad_gather"); }
   }
   p->t += 1;
   float* stat_slot = p->step_stats + 4 * (p->steps_in_epoch % MAX_STEPS_PER_EPOCH);
@@ -451,7 +455,7 @@ TALOS_API talos_status talos_ppo_forward(talos_ppo* p, const float* obs, int64_t
     int64_t m = std::min<int64_t>(c.minibatch, n - s);
     forward(p, obs + s * c.obs_dim, m);
     int64_t total = m * (c.n_actions + 1);
-    unpack_heads_kernel<<<(unsigned)ceil_div(total, 256), 256, 0, p->ctx->stream>>>(p->z, p->HP, c.n_actions, m, logits_out ? logits_out + s * c.n_actions : nullptr,
+    talos_kernel(p->ctx, unpack_heads_kernel, (unsigned)ceil_div(total, 256), 256, 0, p->z, p->HP, c.n_actions, m, logits_out ? logits_out + s * c.n_actions : nullptr,
                                                                                      values_out ? values_out + s : nullptr);
     talos_launched(p->ctx, "unpack_heads");
   }
@@ -464,7 +468,7 @@ TALOS_API talos_status talos_ppo_log_prob(talos_ppo* p, const float* obs, const 
   for (int64_t s = 0; s < n; s += c.minibatch) {
     int64_t m = std::min<int64_t>(c.minibatch, n - s);
     forward(p, obs + s * c.obs_dim, m);
-    log_prob_kernel<<<(unsigned)ceil_div(m, 256), 256, 0, p->ctx->stream>>>(p->z, p->HP, c.n_actions, actions + s, m, out + s, p->ctx->dev_status);
+    talos_kernel(p->ctx, log_prob_kernel, (unsigned)ceil_div(m, 256), 256, 0, p->z, p->HP, c.n_actions, actions + s, m, out + s, p->ctx->dev_status);
     talos_launched(p->ctx, "log_prob");
   }
   TALOS_ENTRY_END

@@ -24,6 +24,7 @@ template <int NVEC>
 __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
 rmsnorm_fwd_vec_kernel(const float4* __restrict__ x, const float4* __restrict__ gamma, float eps, long long rows,
                        int dim4, float* __restrict__ inv_rms, float4* __restrict__ y) {
+  talos_pdl(x, gamma, inv_rms, y);
   const int lane = threadIdx.x & 31;
   const long long warp = (long long)blockIdx.x * WARPS_PER_CTA + (threadIdx.x >> 5);
   const long long nwarps = (long long)gridDim.x * WARPS_PER_CTA;
@@ -58,6 +59,7 @@ rmsnorm_fwd_vec_kernel(const float4* __restrict__ x, const float4* __restrict__ 
 // Any dim / alignment: one warp per row, scalar strided loop, row re-read from cache.
 __global__ void rmsnorm_fwd_generic_kernel(const float* __restrict__ x, const float* __restrict__ gamma, float eps,
                                            long long rows, int dim, float* __restrict__ inv_rms, float* __restrict__ y) {
+  talos_pdl(x, gamma, inv_rms, y);
   const int lane = threadIdx.x & 31;
   const long long warp = (long long)blockIdx.x * WARPS_PER_CTA + (threadIdx.x >> 5);
   const long long nwarps = (long long)gridDim.x * WARPS_PER_CTA;
@@ -78,6 +80,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
 rmsnorm_bwd_kernel(const float* __restrict__ dy, const float* __restrict__ x, const float* __restrict__ gamma,
                    const float* __restrict__ inv_rms, long long rows, int dim, float* __restrict__ dx, int acc_dx,
                    float* __restrict__ partial) {
+  talos_pdl(dy, x, gamma, inv_rms, dx, partial);
   extern __shared__ float sh[];            // [WARPS_PER_CTA][dim] column partials
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   float* mine = sh + (size_t)w * dim;
@@ -112,6 +115,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
 rmsnorm_bwd_vec_kernel(const float4* __restrict__ dy, const float4* __restrict__ x, const float4* __restrict__ gamma,
                        const float* __restrict__ inv_rms, long long rows, int dim4, float4* __restrict__ dx, int acc_dx,
                        float* __restrict__ partial) {
+  talos_pdl(dy, x, gamma, inv_rms, dx, partial);
   extern __shared__ float sh[];            // [WARPS_PER_CTA][dim]
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long long warp = (long long)blockIdx.x * WARPS_PER_CTA + w;
@@ -162,6 +166,7 @@ rmsnorm_bwd_vec_kernel(const float4* __restrict__ dy, const float4* __restrict__
 // lane l sums parts l, l+8, ... then the eight lane sums are added in lane order (deterministic).
 __global__ void __launch_bounds__(256)
 colsum_partials_kernel(const float* __restrict__ partial, int nparts, int dim, float* __restrict__ out, int acc) {
+  talos_pdl(partial, out);
   __shared__ float sh[8][33];
   const int cl = threadIdx.x & 31, pl = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cl;
@@ -183,6 +188,7 @@ colsum_partials_kernel(const float* __restrict__ partial, int nparts, int dim, f
 // Column sums of a [rows, n] matrix, stage 1, any n: each CTA sums a contiguous slab of rows.
 __global__ void colsum_stage1_kernel(const float* __restrict__ g, long long rows, int n, long long rows_per_cta,
                                      float* __restrict__ partial) {
+  talos_pdl(g, partial);
   long long r0 = (long long)blockIdx.y * rows_per_cta, r1 = min(rows, r0 + rows_per_cta);
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
@@ -200,6 +206,7 @@ template <int DACT>
 __global__ void __launch_bounds__(256)
 colsum_stage1_vec_kernel(const float4* g, float4* g_out, const float4* __restrict__ saved, long long rows, int n4, long long rows_per_cta,
                          float* __restrict__ partial) {
+  talos_pdl(g, g_out, saved, partial);
   extern __shared__ float4 shv[];                       // [row_lanes][n4]
   const int row_lanes = 256 / n4;
   const int cl = threadIdx.x % n4, rl = threadIdx.x / n4;
@@ -231,6 +238,7 @@ colsum_stage1_vec_kernel(const float4* g, float4* g_out, const float4* __restric
 template <int NPL>
 __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
 softmax_fwd_kernel(const float* __restrict__ x, float* __restrict__ y, long long rows, int len, float scale, int causal_period) {
+  talos_pdl(x, y);
   const int lane = threadIdx.x & 31;
   const long long warp = (long long)blockIdx.x * WARPS_PER_CTA + (threadIdx.x >> 5);
   const long long nwarps = (long long)gridDim.x * WARPS_PER_CTA;
@@ -272,6 +280,7 @@ template <> __device__ __forceinline__ float4 arr_to_vec<4>(const float* a) { re
 template <int LPR, int NV>
 __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
 softmax_fwd_vec_kernel(const float* __restrict__ x, float* __restrict__ y, long long rows, float scale, int causal_period) {
+  talos_pdl(x, y);
   constexpr int LEN = LPR * 4 * NV, RPW = 32 / LPR;
   const int lane = threadIdx.x & 31, sub = lane / LPR, l = lane % LPR;
   const long long warp = (long long)blockIdx.x * WARPS_PER_CTA + (threadIdx.x >> 5);
@@ -316,6 +325,7 @@ template <int NPL>
 __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
 softmax_bwd_kernel(const float* __restrict__ y, const float* dy, float* dx, long long rows,
                    int len, float scale, int acc) {
+  talos_pdl(y, dy, dx);
   const int lane = threadIdx.x & 31;
   const long long warp = (long long)blockIdx.x * WARPS_PER_CTA + (threadIdx.x >> 5);
   const long long nwarps = (long long)gridDim.x * WARPS_PER_CTA;
@@ -341,6 +351,7 @@ softmax_bwd_kernel(const float* __restrict__ y, const float* dy, float* dx, long
 __global__ void rope_kernel(const float2* __restrict__ x, float2* __restrict__ y, const float* __restrict__ cos_t,
                             const float* __restrict__ sin_t, long long table_len, long long total_pairs, int npos,
                             int inner, int half, long long start_pos, int inverse, int acc) {
+  talos_pdl(x, y, cos_t, sin_t);
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total_pairs) return;
   int i = (int)(idx % half);
@@ -363,6 +374,7 @@ __global__ void __launch_bounds__(256)
 rope_vec_kernel(const float4* __restrict__ x, float4* __restrict__ y, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                 unsigned table_len, unsigned total_quads, unsigned npos, unsigned inner, unsigned quads_per_row, unsigned start_pos,
                 int inverse, int acc) {
+  talos_pdl(x, y, cos_t, sin_t);
   for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total_quads; idx += gridDim.x * blockDim.x) {
     const unsigned qi = idx % quads_per_row, rest = idx / quads_per_row;
     const unsigned p = (rest / inner) % npos;
@@ -401,11 +413,11 @@ TALOS_API talos_status talos_rmsnorm_fwd(talos_ctx* ctx, const float* x, const f
   if (dim % 4 == 0 && dim <= 32 * 4 * MAX_VEC && aligned16(x) && aligned16(y) && aligned16(gamma)) {
     int dim4 = (int)(dim / 4), nvec = (int)ceil_div(dim4, 32);
     auto X = (const float4*)x; auto G = (const float4*)gamma; auto Y = (float4*)y;
-#define TALOS_RMS_CASE(NV) case NV: rmsnorm_fwd_vec_kernel<NV><<<grid, WARPS_PER_CTA * 32, 0, ctx->stream>>>(X, G, eps, rows, dim4, inv_rms, Y); break;
+#define TALOS_RMS_CASE(NV) case NV: talos_kernel(ctx, rmsnorm_fwd_vec_kernel<NV>, grid, WARPS_PER_CTA * 32, 0, X, G, eps, rows, dim4, inv_rms, Y); break;
     switch (nvec) { TALOS_RMS_CASE(1) TALOS_RMS_CASE(2) TALOS_RMS_CASE(3) TALOS_RMS_CASE(4) TALOS_RMS_CASE(5) TALOS_RMS_CASE(6) TALOS_RMS_CASE(7) TALOS_RMS_CASE(8) }
 #undef TALOS_RMS_CASE
   } else {
-    rmsnorm_fwd_generic_kernel<<<grid, WARPS_PER_CTA * 32, 0, ctx->stream>>>(x, gamma, eps, rows, (int)dim, inv_rms, y);
+    talos_kernel(ctx, rmsnorm_fwd_generic_kernel, grid, WARPS_PER_CTA * 32, 0, x, gamma, eps, rows, (int)dim, inv_rms, y);
   }
   talos_launched(ctx, "rmsnorm_fwd");
   TALOS_ENTRY_END
@@ -425,15 +437,15 @@ TALOS_API talos_status talos_rmsnorm_bwd(talos_ctx* ctx, const float* dy, const 
   if (dim % 4 == 0 && dim <= 32 * 4 * MAX_VEC && aligned16(dy) && aligned16(x) && aligned16(gamma) && (!dx || aligned16(dx))) {
     const int dim4 = (int)(dim / 4), nvec = (int)ceil_div(dim4, 32);
     auto DY = (const float4*)dy; auto X = (const float4*)x; auto G = (const float4*)gamma; auto DX = (float4*)dx;
-#define TALOS_RB_CASE(NV) case NV: rmsnorm_bwd_vec_kernel<NV><<<grid, WARPS_PER_CTA * 32, shmem, ctx->stream>>>(DY, X, G, inv_rms, rows, dim4, DX, accumulate & 1, partial); break;
+#define TALOS_RB_CASE(NV) case NV: talos_kernel(ctx, rmsnorm_bwd_vec_kernel<NV>, grid, WARPS_PER_CTA * 32, shmem, DY, X, G, inv_rms, rows, dim4, DX, accumulate & 1, partial); break;
     switch (nvec) { TALOS_RB_CASE(1) TALOS_RB_CASE(2) TALOS_RB_CASE(3) TALOS_RB_CASE(4) TALOS_RB_CASE(5) TALOS_RB_CASE(6) TALOS_RB_CASE(7) TALOS_RB_CASE(8) }
 #undef TALOS_RB_CASE
   } else
-  rmsnorm_bwd_kernel<<<grid, WARPS_PER_CTA * 32, shmem, ctx->stream>>>(dy, x, gamma, inv_rms, rows, (int)dim, dx,
+  talos_kernel(ctx, rmsnorm_bwd_kernel, grid, WARPS_PER_CTA * 32, shmem, dy, x, gamma, inv_rms, rows, (int)dim, dx,
                                                                         accumulate & 1, partial);
   talos_launched(ctx, "rmsnorm_bwd");
   if (dgamma) {
-    colsum_partials_kernel<<<(unsigned)ceil_div(dim, 32), 256, 0, ctx->stream>>>(partial, grid, (int)dim, dgamma, (accumulate >> 1) & 1);
+    talos_kernel(ctx, colsum_partials_kernel, (unsigned)ceil_div(dim, 32), 256, 0, partial, grid, (int)dim, dgamma, (accumulate >> 1) & 1);
     talos_launched(ctx, "rmsnorm_dgamma");
   }
   TALOS_ENTRY_END
@@ -455,15 +467,15 @@ static bool colsum_vec_launch(talos_ctx* ctx, const float* g, float* g_out, cons
   size_t shmem = sizeof(float4) * (size_t)(256 / n4) * n4;
   auto G4 = (const float4*)g; auto O4 = (float4*)g_out; auto S4 = (const float4*)saved;
   switch (dact) {
-    case 0: colsum_stage1_vec_kernel<0><<<(unsigned)slabs, 256, shmem, ctx->stream>>>(G4, O4, S4, rows, n4, rows_per, partial); break;
-    case TALOS_ACT_RELU: colsum_stage1_vec_kernel<TALOS_ACT_RELU><<<(unsigned)slabs, 256, shmem, ctx->stream>>>(G4, O4, S4, rows, n4, rows_per, partial); break;
-    case TALOS_ACT_TANH: colsum_stage1_vec_kernel<TALOS_ACT_TANH><<<(unsigned)slabs, 256, shmem, ctx->stream>>>(G4, O4, S4, rows, n4, rows_per, partial); break;
-    case TALOS_ACT_SILU: colsum_stage1_vec_kernel<TALOS_ACT_SILU><<<(unsigned)slabs, 256, shmem, ctx->stream>>>(G4, O4, S4, rows, n4, rows_per, partial); break;
+    case 0: talos_kernel(ctx, colsum_stage1_vec_kernel<0>, (unsigned)slabs, 256, shmem, G4, O4, S4, rows, n4, rows_per, partial); break;
+    case TALOS_ACT_RELU: talos_kernel(ctx, colsum_stage1_vec_kernel<TALOS_ACT_RELU>, (unsigned)slabs, 256, shmem, G4, O4, S4, rows, n4, rows_per, partial); break;
+    case TALOS_ACT_TANH: talos_kernel(ctx, colsum_stage1_vec_kernel<TALOS_ACT_TANH>, (unsigned)slabs, 256, shmem, G4, O4, S4, rows, n4, rows_per, partial); break;
+    case TALOS_ACT_SILU: talos_kernel(ctx, colsum_stage1_vec_kernel<TALOS_ACT_SILU>, (unsigned)slabs, 256, shmem, G4, O4, S4, rows, n4, rows_per, partial); break;
     default: throw talos_error(TALOS_ERR_ARG, "bad activation kind");
   }
   talos_launched(ctx, "colsum_stage1");
   if (ext_partial) { *slabs_out = (int)slabs; return true; }
-  colsum_partials_kernel<<<(unsigned)ceil_div(n, 32), 256, 0, ctx->stream>>>(partial, (int)slabs, (int)n, out, accumulate ? 1 : 0);
+  talos_kernel(ctx, colsum_partials_kernel, (unsigned)ceil_div(n, 32), 256, 0, partial, (int)slabs, (int)n, out, accumulate ? 1 : 0);
   talos_launched(ctx, "colsum_stage2");
   return true;
 }
@@ -492,9 +504,9 @@ TALOS_API talos_status talos_colsum(talos_ctx* ctx, const float* g, float* out, 
   int64_t slabs = std::max<int64_t>(1, std::min<int64_t>(ceil_div(rows, 64), (4 * (int64_t)ctx->sm_count) / col_blocks + 1));
   int64_t rows_per = std::max<int64_t>(1, ceil_div(rows, slabs)); slabs = std::max<int64_t>(1, ceil_div(rows, rows_per));
   float* partial = (float*)talos_workspace(ctx, sizeof(float) * (size_t)slabs * n);
-  colsum_stage1_kernel<<<dim3((unsigned)col_blocks, (unsigned)slabs), 128, 0, ctx->stream>>>(g, rows, (int)n, rows_per, partial);
+  talos_kernel(ctx, colsum_stage1_kernel, dim3((unsigned)col_blocks, (unsigned)slabs), 128, 0, g, rows, (int)n, rows_per, partial);
   talos_launched(ctx, "colsum_stage1");
-  colsum_partials_kernel<<<(unsigned)ceil_div(n, 32), 256, 0, ctx->stream>>>(partial, (int)slabs, (int)n, out, accumulate ? 1 : 0);
+  talos_kernel(ctx, colsum_partials_kernel, (unsigned)ceil_div(n, 32), 256, 0, partial, (int)slabs, (int)n, out, accumulate ? 1 : 0);
   talos_launched(ctx, "colsum_stage2");
   TALOS_ENTRY_END
 }
@@ -511,16 +523,16 @@ TALOS_API talos_status talos_softmax_fwd(talos_ctx* ctx, const float* x, float* 
   int grid = row_grid(ctx, len <= 128 ? ceil_div(rows, 4) : rows); int npl = (int)ceil_div(len, 32);
   if (aligned16(x) && aligned16(y) && (len == 64 || len == 128 || len == 256 || len == 512)) {
     const int cp = (int)causal_period;
-    if (len == 64) softmax_fwd_vec_kernel<8, 2><<<grid, WARPS_PER_CTA * 32, 0, ctx->stream>>>(x, y, rows, scale, cp);
-    else if (len == 128) softmax_fwd_vec_kernel<8, 4><<<grid, WARPS_PER_CTA * 32, 0, ctx->stream>>>(x, y, rows, scale, cp);
-    else if (len == 256) softmax_fwd_vec_kernel<16, 4><<<grid, WARPS_PER_CTA * 32, 0, ctx->stream>>>(x, y, rows, scale, cp);
-    else softmax_fwd_vec_kernel<32, 4><<<grid, WARPS_PER_CTA * 32, 0, ctx->stream>>>(x, y, rows, scale, cp);
+    if (len == 64) talos_kernel(ctx, softmax_fwd_vec_kernel<8, 2>, grid, WARPS_PER_CTA * 32, 0, x, y, rows, scale, cp);
+    else if (len == 128) talos_kernel(ctx, softmax_fwd_vec_kernel<8, 4>, grid, WARPS_PER_CTA * 32, 0, x, y, rows, scale, cp);
+    else if (len == 256) talos_kernel(ctx, softmax_fwd_vec_kernel<16, 4>, grid, WARPS_PER_CTA * 32, 0, x, y, rows, scale, cp);
+    else talos_kernel(ctx, softmax_fwd_vec_kernel<32, 4>, grid, WARPS_PER_CTA * 32, 0, x, y, rows, scale, cp);
     talos_launched(ctx, "softmax_fwd");
     return TALOS_OK;
   }
-#define TALOS_SM_CASE(NP) if (npl <= NP) softmax_fwd_kernel<NP><<<grid, WARPS_PER_CTA * 32, 0, ctx->stream>>>(x, y, rows, (int)len, scale, (int)causal_period); else
+#define TALOS_SM_CASE(NP) if (npl <= NP) talos_kernel(ctx, softmax_fwd_kernel<NP>, grid, WARPS_PER_CTA * 32, 0, x, y, rows, (int)len, scale, (int)causal_period); else
   TALOS_SM_CASE(1) TALOS_SM_CASE(2) TALOS_SM_CASE(4) TALOS_SM_CASE(8) TALOS_SM_CASE(16)
-  softmax_fwd_kernel<32><<<grid, WARPS_PER_CTA * 32, 0, ctx->stream>>>(x, y, rows, (int)len, scale, (int)causal_period);
+  talos_kernel(ctx, softmax_fwd_kernel<32>, grid, WARPS_PER_CTA * 32, 0, x, y, rows, (int)len, scale, (int)causal_period);
 #undef TALOS_SM_CASE
   talos_launched(ctx, "softmax_fwd");
   TALOS_ENTRY_END
@@ -534,9 +546,9 @@ TALOS_API talos_status talos_softmax_bwd(talos_ctx* ctx, const float* y, const f
   if (rows == 0 || len == 0) return TALOS_OK;
   TALOS_REQUIRE(y && dy && dx, TALOS_ERR_ARG, "null pointer");
   int grid = row_grid(ctx, rows); int npl = (int)ceil_div(len, 32); int acc = accumulate ? 1 : 0;
-#define TALOS_SM_CASE(NP) if (npl <= NP) softmax_bwd_kernel<NP><<<grid, WARPS_PER_CTA * 32, 0, ctx->stream>>>(y, dy, dx, rows, (int)len, scale, acc); else
+#define TALOS_SM_CASE(NP) if (npl <= NP) talos_kernel(ctx, softmax_bwd_kernel<NP>, grid, WARPS_PER_CTA * 32, 0, y, dy, dx, rows, (int)len, scale, acc); else
   TALOS_SM_CASE(1) TALOS_SM_CASE(2) TALOS_SM_CASE(4) TALOS_SM_CASE(8) TALOS_SM_CASE(16)
-  softmax_bwd_kernel<32><<<grid, WARPS_PER_CTA * 32, 0, ctx->stream>>>(y, dy, dx, rows, (int)len, scale, acc);
+  talos_kernel(ctx, softmax_bwd_kernel<32>, grid, WARPS_PER_CTA * 32, 0, y, dy, dx, rows, (int)len, scale, acc);
 #undef TALOS_SM_CASE
   talos_launched(ctx, "softmax_bwd");
   TALOS_ENTRY_END
@@ -576,12 +588,12 @@ TALOS_API talos_status talos_rope(talos_ctx* ctx, const float* x, float* y, cons
       table_len < (1LL << 31) && start_pos + npos < (1LL << 20)) {
     const unsigned quads = (unsigned)(pairs / 2);
     const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(quads, 256), (int64_t)ctx->sm_count * 16);
-    rope_vec_kernel<<<grid, 256, 0, ctx->stream>>>((const float4*)x, (float4*)y, cos_t, sin_t, (unsigned)table_len, quads, (unsigned)npos,
+    talos_kernel(ctx, rope_vec_kernel, grid, 256, 0, (const float4*)x, (float4*)y, cos_t, sin_t, (unsigned)table_len, quads, (unsigned)npos,
                                                    (unsigned)inner, (unsigned)(dim / 4), (unsigned)start_pos, inverse ? 1 : 0, accumulate ? 1 : 0);
     talos_launched(ctx, "rope");
     return TALOS_OK;
   }
-  rope_kernel<<<(unsigned)ceil_div(pairs, 256), 256, 0, ctx->stream>>>((const float2*)x, (float2*)y, cos_t, sin_t, table_len,
+  talos_kernel(ctx, rope_kernel, (unsigned)ceil_div(pairs, 256), 256, 0, (const float2*)x, (float2*)y, cos_t, sin_t, table_len,
                                                                         pairs, (int)npos, (int)inner, (int)(dim / 2), start_pos,
                                                                         inverse ? 1 : 0, accumulate ? 1 : 0);
   talos_launched(ctx, "rope");

@@ -43,6 +43,7 @@ __device__ __forceinline__ float block_max(float v, float* sh) {
 template <int KIND>
 __global__ void __launch_bounds__(THREADS)
 axpy_like_kernel(float* __restrict__ out, const float* __restrict__ a, const float* __restrict__ b, float scale, long long n, int vec) {
+  talos_pdl(out, a, b);
   const long long tid = (long long)blockIdx.x * THREADS + threadIdx.x, nthreads = (long long)gridDim.x * THREADS;
   long long done = 0;
   if (vec) {
@@ -68,6 +69,7 @@ axpy_like_kernel(float* __restrict__ out, const float* __restrict__ a, const flo
 
 __global__ void __launch_bounds__(THREADS)
 dot_stage1_kernel(const float* __restrict__ a, const float* __restrict__ b, long long n, int vec, float* __restrict__ partial) {
+  talos_pdl(a, b, partial);
   __shared__ float sh[THREADS / 32];
   const long long tid = (long long)blockIdx.x * THREADS + threadIdx.x, nthreads = (long long)gridDim.x * THREADS;
   float s = 0.f; long long done = 0;
@@ -86,6 +88,7 @@ dot_stage1_kernel(const float* __restrict__ a, const float* __restrict__ b, long
 // One block adds the stage-1 partials (strided, then the fixed shuffle tree) and writes / accumulates the scalar.
 __global__ void __launch_bounds__(THREADS)
 sum_partials_kernel(const float* __restrict__ partial, int nparts, float* __restrict__ out, int accumulate) {
+  talos_pdl(partial, out);
   __shared__ float sh[THREADS / 32];
   float s = 0.f;
   for (int i = threadIdx.x; i < nparts; i += THREADS) s += partial[i];
@@ -95,6 +98,7 @@ sum_partials_kernel(const float* __restrict__ partial, int nparts, float* __rest
 
 __global__ void __launch_bounds__(THREADS)
 max_stage1_kernel(const float* __restrict__ x, long long n, float* __restrict__ partial) {
+  talos_pdl(x, partial);
   __shared__ float sh[THREADS / 32];
   float m = -INFINITY;
   for (long long i = (long long)blockIdx.x * THREADS + threadIdx.x; i < n; i += (long long)gridDim.x * THREADS) m = fmaxf(m, x[i]);
@@ -104,6 +108,7 @@ max_stage1_kernel(const float* __restrict__ x, long long n, float* __restrict__ 
 // row[i] = exp(row[i] - max); per-block sums of the results.  Every block first reduces the (few) per-block maxima.
 __global__ void __launch_bounds__(THREADS)
 exp_sum_stage2_kernel(float* __restrict__ x, long long n, const float* __restrict__ max_partial, int nparts, float* __restrict__ sum_partial) {
+  talos_pdl(x, max_partial, sum_partial);
   __shared__ float sh[THREADS / 32];
   __shared__ float mx_s;
   float m = -INFINITY;
@@ -135,7 +140,7 @@ TALOS_API talos_status talos_axpy(talos_ctx* ctx, float* out, const float* row, 
   TALOS_REQUIRE(n >= 0, TALOS_ERR_SHAPE, "Dimension mismatch in add_scaled_row");
   if (n == 0) return TALOS_OK;
   TALOS_REQUIRE(out && row, TALOS_ERR_ARG, "null pointer");
-  axpy_like_kernel<0><<<blocks_for(ctx, n, 8), THREADS, 0, ctx->stream>>>(out, row, nullptr, scale, n, aligned16(out, row) ? 1 : 0);
+  talos_kernel(ctx, axpy_like_kernel<0>, blocks_for(ctx, n, 8), THREADS, 0, out, row, nullptr, scale, n, aligned16(out, row) ? 1 : 0);
   talos_launched(ctx, "axpy");
   TALOS_ENTRY_END
 }
@@ -146,7 +151,7 @@ TALOS_API talos_status talos_vector_fma(talos_ctx* ctx, float* dst, const float*
   TALOS_REQUIRE(n >= 0, TALOS_ERR_SHAPE, "bad length");
   if (n == 0) return TALOS_OK;
   TALOS_REQUIRE(dst && a && b, TALOS_ERR_ARG, "null pointer");
-  axpy_like_kernel<1><<<blocks_for(ctx, n, 8), THREADS, 0, ctx->stream>>>(dst, a, b, 0.f, n, aligned16(dst, a, b) ? 1 : 0);
+  talos_kernel(ctx, axpy_like_kernel<1>, blocks_for(ctx, n, 8), THREADS, 0, dst, a, b, 0.f, n, aligned16(dst, a, b) ? 1 : 0);
   talos_launched(ctx, "vector_fma");
   TALOS_ENTRY_END
 }
@@ -157,7 +162,7 @@ TALOS_API talos_status talos_vector_scale(talos_ctx* ctx, float* row, float scal
   TALOS_REQUIRE(n >= 0, TALOS_ERR_SHAPE, "bad length");
   if (n == 0) return TALOS_OK;
   TALOS_REQUIRE(row != nullptr, TALOS_ERR_ARG, "null pointer");
-  axpy_like_kernel<2><<<blocks_for(ctx, n, 8), THREADS, 0, ctx->stream>>>(row, nullptr, nullptr, scale, n, aligned16(row) ? 1 : 0);
+  talos_kernel(ctx, axpy_like_kernel<2>, blocks_for(ctx, n, 8), THREADS, 0, row, nullptr, nullptr, scale, n, aligned16(row) ? 1 : 0);
   talos_launched(ctx, "vector_scale");
   TALOS_ENTRY_END
 }
@@ -169,9 +174,9 @@ TALOS_API talos_status talos_dot(talos_ctx* ctx, const float* a, const float* b,
   TALOS_REQUIRE(out != nullptr && ((a && b) || n == 0), TALOS_ERR_ARG, "null pointer");
   const int blocks = blocks_for(ctx, n, 16);
   float* partial = (float*)talos_workspace(ctx, sizeof(float) * MAX_BLOCKS);
-  dot_stage1_kernel<<<blocks, THREADS, 0, ctx->stream>>>(a, b, n, aligned16(a, b) ? 1 : 0, partial);
+  talos_kernel(ctx, dot_stage1_kernel, blocks, THREADS, 0, a, b, n, aligned16(a, b) ? 1 : 0, partial);
   talos_launched(ctx, "dot_stage1");
-  sum_partials_kernel<<<1, THREADS, 0, ctx->stream>>>(partial, blocks, out, accumulate ? 1 : 0);
+  talos_kernel(ctx, sum_partials_kernel, 1, THREADS, 0, partial, blocks, out, accumulate ? 1 : 0);
   talos_launched(ctx, "dot_stage2");
   TALOS_ENTRY_END
 }
@@ -184,11 +189,11 @@ TALOS_API talos_status talos_softmax_exp_sum(talos_ctx* ctx, float* row, int64_t
   if (n == 0) { TALOS_CHECK_CUDA(cudaMemsetAsync(sum_out, 0, sizeof(float), ctx->stream)); return TALOS_OK; }   // empty row: 0.0 (:336-338)
   const int blocks = blocks_for(ctx, n, 8);
   float* partial = (float*)talos_workspace(ctx, sizeof(float) * 2 * MAX_BLOCKS);
-  max_stage1_kernel<<<blocks, THREADS, 0, ctx->stream>>>(row, n, partial);
+  talos_kernel(ctx, max_stage1_kernel, blocks, THREADS, 0, row, n, partial);
   talos_launched(ctx, "exp_sum_max");
-  exp_sum_stage2_kernel<<<blocks, THREADS, 0, ctx->stream>>>(row, n, partial, blocks, partial + MAX_BLOCKS);
+  talos_kernel(ctx, exp_sum_stage2_kernel, blocks, THREADS, 0, row, n, partial, blocks, partial + MAX_BLOCKS);
   talos_launched(ctx, "exp_sum_exp");
-  sum_partials_kernel<<<1, THREADS, 0, ctx->stream>>>(partial + MAX_BLOCKS, blocks, sum_out, 0);
+  talos_kernel(ctx, sum_partials_kernel, 1, THREADS, 0, partial + MAX_BLOCKS, blocks, sum_out, 0);
   talos_launched(ctx, "exp_sum_sum");
   TALOS_ENTRY_END
 }

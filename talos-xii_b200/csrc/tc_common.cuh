@@ -189,7 +189,7 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes
 template <int ACT, int DACT>
 __device__ __forceinline__ void epilogue_rows_t(const EpiArgs& e, const float* stage, int lane, long long m0, int rows_valid,
                                                 long long n, bool col_ok, float* C, long long ldc) {
-  const float bias_v = (e.bias && col_ok) ? __ldg(e.bias + n) : 0.f;
+  const float bias_v = (e.bias && col_ok) ? e.bias[n] : 0.f;
 #pragma unroll 4
   for (int rr = 0; rr < rows_valid; ++rr) {
     if (!col_ok) continue;
@@ -197,7 +197,7 @@ __device__ __forceinline__ void epilogue_rows_t(const EpiArgs& e, const float* s
     float v = stage[rr * 32 + (lane ^ rr)] + bias_v;
     if (e.aux_out) e.aux_out[m * e.ld_aux_out + n] = v;
     if (ACT) v = talos_act(v, ACT);
-    if (DACT) v *= talos_dact(__ldg(e.aux_in + m * e.ld_aux_in + n), DACT);
+    if (DACT) v *= talos_dact(e.aux_in[m * e.ld_aux_in + n], DACT);
     if (e.beta) v += C[m * ldc + n];
     C[m * ldc + n] = v;
   }
@@ -224,10 +224,10 @@ __device__ __noinline__ void epilogue_rows(const EpiArgs e, const float* stage, 
 template <int ACT, int DACT>
 __device__ __forceinline__ float4 epilogue_group(float4 v, const float* __restrict__ bias, const float* __restrict__ aux_in,
                                                  const float* __restrict__ c_old) {
-  if (bias) { const float4 b = __ldg((const float4*)bias); v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w; }
+  if (bias) { const float4 b = *(const float4*)bias; v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w; }
   if (ACT) { v.x = talos_act(v.x, ACT); v.y = talos_act(v.y, ACT); v.z = talos_act(v.z, ACT); v.w = talos_act(v.w, ACT); }
   if (DACT) {
-    const float4 a = __ldg((const float4*)aux_in);
+    const float4 a = *(const float4*)aux_in;
     v.x *= talos_dact(a.x, DACT); v.y *= talos_dact(a.y, DACT); v.z *= talos_dact(a.z, DACT); v.w *= talos_dact(a.w, DACT);
   }
   if (c_old) { const float4 o = *(const float4*)c_old; v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w; }
@@ -323,7 +323,7 @@ if (fuse && c < groups) {                                                       
 #define TALOS_EPI_STRAIGHT(A, HAS_BIAS)                                                                                 \
   { const float4* bp = (const float4*)(g.epi.bias + n0);                                                                \
     _Pragma("unroll") for (int c = 0; c < 8; ++c) {                                                                    \
-      const float4 b4 = HAS_BIAS ? __ldg(bp + c) : make_float4(0.f, 0.f, 0.f, 0.f);                                     \
+      const float4 b4 = HAS_BIAS ? bp[c] : make_float4(0.f, 0.f, 0.f, 0.f);                                     \
       r[4 * c] = __float_as_uint(talos_act(__uint_as_float(r[4 * c]) + b4.x, A));                                       \
       r[4 * c + 1] = __float_as_uint(talos_act(__uint_as_float(r[4 * c + 1]) + b4.y, A));                               \
       r[4 * c + 2] = __float_as_uint(talos_act(__uint_as_float(r[4 * c + 2]) + b4.z, A));                               \

@@ -4,6 +4,7 @@
 #include <vector>
 
 #include "comm.cuh"
+#include "ppo_small.cuh"
 
 // internal launchers of other translation units
 void talos_adam_launch(talos_ctx* ctx, float* p, const float* g, float* m, float* v, int64_t n, int64_t t, float lr, float b1,
@@ -24,6 +25,7 @@ struct talos_ppo {
   // bias gradients stay here until ONE kernel reduces all six into the flat gradient buffer.
   float* partials = nullptr; int64_t cap_w2 = 0, cap_w1 = 0, cap_wh = 0, cap_b = 0;
   float* loss_part = nullptr; int64_t cap_loss = 0;   // loss kernel's per-block partials: [blocks][2] {loss, kl} then [blocks][HP] column sums
+  int small_cluster = 0;               // > 0: policy and minibatch are small enough for the one-launch kernels of ppo_small.cu
   int64_t t = 0; int64_t steps_in_epoch = 0; int64_t last_launches = 0;
   std::vector<float> host_tmp;
   cudaStream_t copy_stream = nullptr;  // host->device staging of talos_ppo_update_host, overlapped with the steps
@@ -33,6 +35,9 @@ struct talos_ppo {
 namespace {
 
 constexpr int MAX_STEPS_PER_EPOCH = 4096;
+// Up to here one cluster beats a launch per product over the whole chip: a step costs 4 us and 5.3 us for every 256 rows (12 us at
+// 256, 50 at 2 048, 92 at 4 096), the launches 80 to 85 us at any of these sizes.
+constexpr int64_t PPO_SMALL_MAX_MINIBATCH = 2048;
 
 void gemm(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, const float* B,
           int64_t ldb, float* C, int64_t ldc, int mode, const EpiArgs& e) {
@@ -129,6 +134,26 @@ __global__ void log_prob_kernel(const float* __restrict__ z, int HP, int A, cons
   out[i] = l[act] - (logf(se) + mx);
 }
 
+PpoSmallNet small_net(const talos_ppo* p) {
+  const auto& c = p->cfg;
+  return PpoSmallNet{p->params, c.obs_dim, c.hidden, c.n_actions, (int)p->n_int, (int)p->o_w1, (int)p->o_b1, (int)p->o_w2, (int)p->o_b2, (int)p->o_wh, (int)p->o_bh};
+}
+// `epochs` passes over N transitions without the host in between; only a single rank's gradients can stay in the cluster.
+void small_steps(talos_ppo* p, const float* obs, const int32_t* actions, const float* old_logp, const float* adv, const float* ret, int64_t N, int32_t epochs) {
+  const auto& c = p->cfg;
+  const int64_t steps = (N + c.minibatch - 1) / c.minibatch * epochs;
+  PpoSmallUpdate a{};
+  a.net = small_net(p); a.obs = obs; a.actions = actions; a.old_logp = old_logp; a.adv = adv; a.ret = ret;
+  a.N = N; a.mb = c.minibatch; a.epochs = epochs;
+  a.params = p->params; a.m = p->m; a.v = p->v; a.grads = p->grads;
+  a.stats = p->step_stats; a.stats_at = (int)(p->steps_in_epoch % MAX_STEPS_PER_EPOCH); a.stats_slots = MAX_STEPS_PER_EPOCH;
+  a.clip = c.clip; a.c_value = c.c_value; a.c_entropy = c.c_entropy; a.lr = c.lr; a.b1 = c.beta1; a.b2 = c.beta2; a.eps = c.eps;
+  a.b1_t = pow((double)c.beta1, (double)p->t); a.b2_t = pow((double)c.beta2, (double)p->t);
+  a.status = p->ctx->dev_status;
+  talos_ppo_small_update_launch(p->ctx, p->small_cluster, a);
+  p->t += steps; p->steps_in_epoch += steps; p->weights_prepared = false; p->last_launches = 1;
+}
+
 void forward(talos_ppo* p, const float* obs, int64_t n) {
   const auto& c = p->cfg; const float* P = p->params;
   ensure_weights_prepared(p);
@@ -176,6 +201,7 @@ void check(talos_ppo* p) { TALOS_REQUIRE(p != nullptr, TALOS_ERR_ARG, "null trai
 
 void step(talos_ppo* p, talos_comm* comm, const float* obs, const int32_t* actions, const float* old_logp, const float* adv,
           const float* ret, int64_t n) {
+  if (p->small_cluster && !comm) { small_steps(p, obs, actions, old_logp, adv, ret, n, 1); return; }
   const auto& c = p->cfg; talos_ctx* ctx = p->ctx; const float* P = p->params;
   // With the peer-memory exchange the step's gradient buffer IS this rank's exchange slot: the backward products write
   // straight into memory the other ranks have mapped, and one kernel does exchange + Adam + weight preparation.
@@ -312,9 +338,16 @@ void update(talos_ppo* p, talos_comm* comm, const float* obs, const int32_t* act
     return cnt > 0 ? (float)(kl / cnt) : 0.f;
   };
   p->steps_in_epoch = 0;
+  const bool small = p->small_cluster && !comm;
   for (int32_t e = 0; e < epochs; ++e) {
     if (!defer) p->steps_in_epoch = 0;                       // (deferred: the slots of later epochs follow the earlier ones)
-    for (int64_t s = 0; s < N; s += mb) {
+    if (small && !(ready && e == 0)) {
+      // one launch an epoch; all that are left where nothing is read back in between (a first epoch still being
+      // copied in goes minibatch by minibatch below)
+      const int32_t passes = defer ? epochs - e : 1;
+      small_steps(p, obs, actions, old_logp, adv, ret, N, passes);
+      e += passes - 1;
+    } else for (int64_t s = 0; s < N; s += mb) {
       int64_t n = std::min(mb, N - s);
       if (ready && e == 0) TALOS_CHECK_CUDA(cudaStreamWaitEvent(p->ctx->stream, (*ready)[(size_t)(s / mb)], 0));
       step(p, comm, obs + s * p->cfg.obs_dim, actions + s, old_logp + s, adv + s, ret + s, n);
@@ -367,6 +400,7 @@ TALOS_API talos_status talos_ppo_create(talos_ctx* ctx, const talos_ppo_config* 
   alloc(&p->z, mb * p->HP); alloc(&p->dz, mb * p->HP);
   alloc(&p->step_stats, 4 * MAX_STEPS_PER_EPOCH);
   p->cap_loss = up4(ceil_div(mb, 128) * (2 + p->HP)); alloc(&p->loss_part, p->cap_loss);
+  if (O <= PPO_SMALL_MAX && H <= PPO_SMALL_MAX && p->HP == PPO_SMALL_HEADS && mb <= PPO_SMALL_MAX_MINIBATCH) p->small_cluster = talos_ppo_small_cluster(ctx);
   if (cfg->mode != TALOS_MODE_FP32) {
     alloc(&p->w_hi, p->n_int);
     if (cfg->mode == TALOS_MODE_TF32X3) alloc(&p->w_lo, p->n_int);
@@ -451,6 +485,7 @@ TALOS_API talos_status talos_ppo_forward(talos_ppo* p, const float* obs, int64_t
   TALOS_ENTRY_BEGIN
   check(p); TALOS_REQUIRE(n >= 0 && (obs || n == 0), TALOS_ERR_ARG, "bad observations");
   const auto& c = p->cfg;
+  if (p->small_cluster) { talos_ppo_small_forward_launch(p->ctx, small_net(p), obs, nullptr, n, nullptr, logits_out, values_out); return TALOS_OK; }
   for (int64_t s = 0; s < n; s += c.minibatch) {
     int64_t m = std::min<int64_t>(c.minibatch, n - s);
     forward(p, obs + s * c.obs_dim, m);
@@ -465,6 +500,7 @@ TALOS_API talos_status talos_ppo_log_prob(talos_ppo* p, const float* obs, const 
   TALOS_ENTRY_BEGIN
   check(p); TALOS_REQUIRE(n >= 0 && ((obs && actions && out) || n == 0), TALOS_ERR_ARG, "null pointer");
   const auto& c = p->cfg;
+  if (p->small_cluster) { talos_ppo_small_forward_launch(p->ctx, small_net(p), obs, actions, n, out, nullptr, nullptr); return TALOS_OK; }
   for (int64_t s = 0; s < n; s += c.minibatch) {
     int64_t m = std::min<int64_t>(c.minibatch, n - s);
     forward(p, obs + s * c.obs_dim, m);

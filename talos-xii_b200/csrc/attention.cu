@@ -3,6 +3,8 @@
 // round trip of the scores through HBM.  Q and K may each be given as two strided sources (a content
 // part and a rotary part) so that MLA's concat + transpose + reshape chain
 // (src/transformer.rs:508-533) never materialises.
+#include <initializer_list>
+
 #include "common.cuh"
 
 // A [batch, head, seq, d] view of strided memory: element (b,h,s,c) = p[b*sb + h*sh + s*ss + c].
@@ -136,10 +138,20 @@ void talos_attention_launch(talos_ctx* ctx, HeadView q1, HeadView q2, HeadView k
 bool talos_attention_tc_fused(talos_ctx* ctx, const float* q, const float* k, const float* v, float* out, float* probs, int64_t BH,
                               int64_t S, int64_t dqk, int64_t dv, float scale, int causal);
 
+bool talos_attention_short_takes(talos_ctx* ctx, int64_t BH, int64_t S, int64_t dqk, int64_t dv, int mode, std::initializer_list<const void*> heads);
+void talos_attention_short_fwd(talos_ctx* ctx, const float* q, const float* k, const float* v, float* out, float* probs, int64_t BH, int64_t S, int64_t dqk, int64_t dv,
+                               float scale, int causal);
+void talos_attention_short_bwd(talos_ctx* ctx, const float* q, const float* k, const float* v, const float* probs, const float* dout, float* dq, float* dk, float* dv, int64_t BH,
+                               int64_t S, int64_t dqk, int64_t dvd, float scale);
+
 static bool attention_fwd_tc(talos_ctx* ctx, const float* q, const float* k, const float* v, float* out, float* probs,
                              int64_t BH, int64_t S, int64_t dqk, int64_t dv, float scale, int causal, int mode) {
   // fast mode, S <= 128: one fused kernel with the scores in tensor memory (attention_tc.cu)
   if (mode == TALOS_MODE_TF32 && talos_attention_tc_fused(ctx, q, k, v, out, probs, BH, S, dqk, dv, scale, causal)) return true;
+  if (!(talos_switches() & SW_ATTN_NO_FUSED) && talos_attention_short_takes(ctx, BH, S, dqk, dv, mode, {q, k, v, out})) {
+    talos_attention_short_fwd(ctx, q, k, v, out, probs, BH, S, dqk, dv, scale, causal);
+    return true;
+  }
   if (S > 1024) return false;                                       // row softmax limit
   float* sc = probs ? probs : (float*)talos_workspace2(ctx, sizeof(float) * (size_t)(BH * S * S));
   const EpiArgs none = talos_epi_args(nullptr);
@@ -162,6 +174,10 @@ TALOS_API talos_status talos_attention_fwd(talos_ctx* ctx, const float* q, const
   if (BH == 0 || S == 0) return TALOS_OK;
   TALOS_REQUIRE(q && k && v && out, TALOS_ERR_ARG, "null pointer");
   if (mode != TALOS_MODE_FP32 && attention_fwd_tc(ctx, q, k, v, out, probs, BH, S, dqk, dv, scale, causal ? 1 : 0, mode)) return TALOS_OK;
+  if (mode == TALOS_MODE_FP32 && !(talos_switches() & SW_ATTN_NO_FUSED) && talos_attention_short_takes(ctx, BH, S, dqk, dv, mode, {q, k, v, out})) {
+    talos_attention_short_fwd(ctx, q, k, v, out, probs, BH, S, dqk, dv, scale, causal ? 1 : 0);
+    return TALOS_OK;
+  }
   HeadView none{nullptr, 0, 0, 0, 0};
   talos_attention_launch(ctx, HeadView{q, S * dqk, 0, dqk, (int)dqk}, none, HeadView{k, S * dqk, 0, dqk, (int)dqk}, none,
                          HeadView{v, S * dv, 0, dv, (int)dv}, HeadViewOut{out, S * dv, 0, dv, (int)dv}, probs, BH, 1, (int)S,
@@ -182,6 +198,10 @@ TALOS_API talos_status talos_attention_bwd(talos_ctx* ctx, const float* q, const
   TALOS_REQUIRE(mode >= TALOS_MODE_FP32 && mode <= TALOS_MODE_TF32, TALOS_ERR_ARG, "bad arithmetic mode");
   if (BH == 0 || S == 0) return TALOS_OK;
   TALOS_REQUIRE(q && k && v && probs && dout && dq && dk && dv, TALOS_ERR_ARG, "null pointer");
+  if (!(talos_switches() & SW_ATTN_NO_FUSED) && talos_attention_short_takes(ctx, BH, S, dqk, dvd, mode, {q, k, v, dout, dq, dk, dv})) {
+    talos_attention_short_bwd(ctx, q, k, v, probs, dout, dq, dk, dv, BH, S, dqk, dvd, scale);
+    return TALOS_OK;
+  }
   float* dS = (float*)talos_workspace2(ctx, sizeof(float) * (size_t)(BH * S * S));
   talos_status st;
   st = talos_gemm_batched(ctx, TALOS_OP_T, TALOS_OP_N, S, dvd, S, probs, S, S * S, dout, dvd, S * dvd, dv, dvd, S * dvd, BH, 0, mode);

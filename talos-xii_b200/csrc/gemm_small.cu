@@ -123,6 +123,7 @@ struct SmallTile {
 template <int BM, int BN, int TM, int KG, int KC>
 struct SmallCfg {
   static constexpr int TN = 4, GT = (BM / TM) * (BN / TN), T = GT * KG, PA = BM + 4, PB = BN + 4, BUF = KC * (PA + PB);
+  static constexpr int CTAS = T <= 256 ? 3 : BM <= 32 ? 2 : 1;        // resident on an SM at least
   static constexpr int STAGE = 2 * BUF, SUMS = (KG + 1) * BM * BN + T + BN, BYTES = 4 * (STAGE > SUMS ? STAGE : SUMS);   // two chunks, later the groups' sums, column sums and the partial tile
 };
 template <int BM, int BN, int TM, int KG, int KC, bool VEC, bool DACT>
@@ -243,7 +244,7 @@ __device__ __forceinline__ void small_product(const SmallProduct& g, unsigned it
 }
 
 template <int BM, int BN, int TM, int KG, int KC, bool VEC>
-__global__ void __launch_bounds__((SmallCfg<BM, BN, TM, KG, KC>::T), (BM <= 32 ? 2 : 1))
+__global__ void __launch_bounds__((SmallCfg<BM, BN, TM, KG, KC>::T), (SmallCfg<BM, BN, TM, KG, KC>::CTAS))
 gemm_small_kernel(const __grid_constant__ SmallProduct g) {
   talos_pdl();
   extern __shared__ __align__(16) float sm[];
@@ -266,21 +267,21 @@ bool small_vec(const SmallOperand& o, int64_t rows, int64_t K) {
 }
 // Tiles, and the split of the reduction: as many CTAs as it has chunks while every SM has a slot for them, at most the
 // eight of a portable cluster (adding up the partial tiles takes about as long as one chunk).
-void small_shape(talos_ctx* ctx, SmallProduct& g, int bm, int kc, int64_t batch, int64_t slots) {
-  g.m_tiles = (int)ceil_div(g.M, bm); g.n_tiles = (int)ceil_div(g.N, bm); g.batch = (int)batch;
+void small_shape(talos_ctx* ctx, SmallProduct& g, int bm, int bn, int kc, int64_t batch, int64_t slots) {
+  g.m_tiles = (int)ceil_div(g.M, bm); g.n_tiles = (int)ceil_div(g.N, bn); g.batch = (int)batch;
   const int64_t tiles = (int64_t)g.m_tiles * g.n_tiles * batch, chunks = std::max<int64_t>(1, ceil_div(g.K, kc));
   int splits = 1;
   while (splits < 8 && splits < chunks && tiles * splits * 2 <= slots) splits *= 2;
   g.splits = splits; g.k_split = (int)(ceil_div(chunks, splits) * kc);
 }
 int small_tile(talos_ctx* ctx, int64_t tiles16, int64_t tiles32) { return tiles16 <= 2 * ctx->sm_count ? 16 : tiles32 <= 2 * ctx->sm_count ? 32 : 64; }
-template <int BM, int TM, int KG, int KC, bool VEC>
-void launch_gemm(talos_ctx* ctx, SmallProduct& g, int64_t batch, int64_t slots) {
-  using Cfg = SmallCfg<BM, BM, TM, KG, KC>;
-  small_shape(ctx, g, BM, KC, batch, slots);
+template <int BM, int BN, int TM, int KG, int KC, bool VEC>
+void launch_gemm(talos_ctx* ctx, SmallProduct& g, int64_t batch) {
+  using Cfg = SmallCfg<BM, BN, TM, KG, KC>;
+  small_shape(ctx, g, BM, BN, KC, batch, Cfg::CTAS * (int64_t)ctx->sm_count);
   static std::atomic<uint64_t> smem_set{0};
-  talos_allow_smem(smem_set, (const void*)gemm_small_kernel<BM, BM, TM, KG, KC, VEC>, Cfg::BYTES, ctx->device);
-  talos_kernel_cluster(ctx, gemm_small_kernel<BM, BM, TM, KG, KC, VEC>, (unsigned)((int64_t)g.m_tiles * g.n_tiles * batch * g.splits), Cfg::T, Cfg::BYTES, g.splits, g);
+  talos_allow_smem(smem_set, (const void*)gemm_small_kernel<BM, BN, TM, KG, KC, VEC>, Cfg::BYTES, ctx->device);
+  talos_kernel_cluster(ctx, gemm_small_kernel<BM, BN, TM, KG, KC, VEC>, (unsigned)((int64_t)g.m_tiles * g.n_tiles * batch * g.splits), Cfg::T, Cfg::BYTES, g.splits, g);
 }
 template <int BM, int TM, int KG, int KC, bool VEC>
 void launch_bwd(talos_ctx* ctx, SmallProduct& gx, SmallProduct& gw, int64_t slots) {
@@ -289,9 +290,9 @@ void launch_bwd(talos_ctx* ctx, SmallProduct& gx, SmallProduct& gw, int64_t slot
   gx.splits = gw.splits = 1;
   if (gw.C) {       // the longer reduction: it gets what dX's tiles leave
     const int64_t tiles_x = gx.C ? ceil_div(gx.M, BM) * ceil_div(gx.N, BM) : 0;
-    small_shape(ctx, gw, BM, KC, 1, std::max(slots - tiles_x, slots / 2)); items_w = (int64_t)gw.m_tiles * gw.n_tiles * gw.splits;
+    small_shape(ctx, gw, BM, BM, KC, 1, std::max(slots - tiles_x, slots / 2)); items_w = (int64_t)gw.m_tiles * gw.n_tiles * gw.splits;
   }
-  if (gx.C) { small_shape(ctx, gx, BM, KC, 1, slots - items_w); items_x = (int64_t)gx.m_tiles * gx.n_tiles * gx.splits; }
+  if (gx.C) { small_shape(ctx, gx, BM, BM, KC, 1, slots - items_w); items_x = (int64_t)gx.m_tiles * gx.n_tiles * gx.splits; }
   const int cluster = std::max(gx.splits, gw.splits);
   items_w = ceil_div(items_w, cluster) * cluster;
   static std::atomic<uint64_t> smem_set{0};
@@ -314,10 +315,16 @@ void talos_gemm_small_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_
   // The tile is the smallest that leaves the product in one round of CTAs (two of the smaller ones fit an SM): an SM's fp32 units
   // take 1 024 cycles for a chunk of a 32 x 32 tile and a quarter of that for a 16 x 16 one, which is what is left once
   // the launch and the loads are as short as they get; larger tiles re-read the operands less often.
-#define TALOS_SMALL(BM, TM, KG, KC) { if (vec) launch_gemm<BM, TM, KG, KC, true>(ctx, g, batch, slots); else launch_gemm<BM, TM, KG, KC, false>(ctx, g, batch, slots); }
+#define TALOS_SMALL(BM, BN, TM, KG, KC) { if (vec) launch_gemm<BM, BN, TM, KG, KC, true>(ctx, g, batch); else launch_gemm<BM, BN, TM, KG, KC, false>(ctx, g, batch); }
+  // Past one round, three CTAs of 256 threads an SM hide each other's loads and stores: a narrow result (a head's logits) takes
+  // 64 x 16 tiles (65 536 x 5 x 64: 31 -> 13 us, 20 000 x 5 x 64: 13.5 -> 5.9), a short reduction tiles whose k range is not
+  // shared out, since those sums cost more than 64 products do (65 536 x 64 x 8: 18 -> 9.1 us, 8 192 x 256 x 16: 11.3 -> 7.4; within
+  // one round the shared-out range stays ahead, 1 200 x 256 x 64: 5.4 against 8.6, and so do 32 x 32 tiles, 8 192 x 16 x 256: 9.7
+  // against 11.3).
   const int tile = small_tile(ctx, ceil_div(M, 16) * ceil_div(N, 16) * batch, ceil_div(M, 32) * ceil_div(N, 32) * batch);
-  const int64_t slots = (tile == 64 ? 1 : 2) * (int64_t)ctx->sm_count;
-  if (tile == 16) TALOS_SMALL(16, 2, 16, 128) else if (tile == 32) TALOS_SMALL(32, 4, 8, 128) else TALOS_SMALL(64, 8, 4, 64)
+  const bool rounds = ceil_div(M, 64) * ceil_div(N, 64) * batch > ctx->sm_count;
+  if (tile == 16) TALOS_SMALL(16, 16, 2, 16, 128) else if (tile == 32) TALOS_SMALL(32, 32, 4, 8, 128) else if (N <= 16) TALOS_SMALL(64, 16, 4, 4, 64)
+  else if (K <= 64 && rounds) TALOS_SMALL(64, 64, 4, 1, 32) else TALOS_SMALL(64, 64, 8, 4, 64)
 #undef TALOS_SMALL
   talos_launched(ctx, "gemm_small");
 }

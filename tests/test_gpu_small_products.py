@@ -20,7 +20,7 @@ def ctx(talos):
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 1, 1), (15, 17, 5), (16, 16, 128), (33, 31, 129), (64, 64, 64), (65, 4, 300), (40, 36, 1100), (1000, 64, 20),
-                                   (2100, 68, 33), (17, 2000, 8), (200, 200, 1025)])
+                                   (2100, 68, 33), (17, 2000, 8), (200, 200, 1025), (9500, 5, 70), (9600, 16, 64), (9700, 65, 33), (9600, 64, 64)])
 @pytest.mark.parametrize("opA,opB", [(0, 0), (0, 1), (1, 0), (1, 1)])
 def test_product(talos, ctx, M, N, K, opA, opB):
     import torch

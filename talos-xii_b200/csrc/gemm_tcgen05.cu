@@ -490,6 +490,7 @@ void launch_major(talos_ctx* ctx, bool a_mn, bool b_mn, const CUtensorMap& ta, c
 
 static inline bool x3_mode(int mode) { return mode == TALOS_MODE_TF32X3; }
 thread_local bool g_check_fold = false;   // set by the self-check: the whole reduction in one item, so that its 17 k-blocks are two chains folded on chip
+thread_local bool g_check_width = false;  // set by the self-check so that its few rows still exercise the widest tiles
 thread_local bool g_check_pair = false;   // set by the start-up self-check so that its short reduction still exercises the pair kernel
 
 // A batched product: `batch` independent GEMMs whose operands are `stride*` elements apart (batch 1: a plain GEMM).
@@ -510,6 +511,11 @@ void tc_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K
   if (short_k) bn = 128;
   // (that configuration is all epilogue: sixteen epilogue warps, one 32-column chunk of a tile each, instead of eight with two)
   const bool wide_epi = short_k && !(sw & SW_TC_NO_WIDE_EPI);
+  // Few row panels and a reduction too short to split: narrower tiles as long as each still has an SM of its own.  The
+  // products of 8 192 x 256 x 256 otherwise leave 84 of 148 SMs idle while 64 run twice the columns (three-layer network
+  // 64-256-256-16 on 8 192 rows, forward and backward: 180 -> 169 us).  The fused tanh' epilogue is built for 256 columns.
+  if (!batched && !short_k && K < 16 * BK && !(extra && extra->tanh_saved) && !g_check_width && !(sw & SW_TC_FORCE_PAIR))
+    while (bn > 64 && ceil_div(M, BM) * ceil_div(N, bn / 2) <= ctx->sm_count) bn /= 2;
   TcArgs g;
   g.M = (int)M; g.N = (int)N; g.K = (int)K; g.C = C; g.ldc = ldc; g.epi = epi; g.status = ctx->dev_status; g.partial = nullptr;
   g.batch = (int)std::max<int64_t>(bt.batch, 1); g.stride_c = batched ? bt.stride_c : 0;
@@ -747,13 +753,14 @@ bool self_check_shape(talos_ctx* ctx, const int M, const int N = 328, const int 
 // reduction longer than one accumulation chain); then a batch
 // of three small ragged products (tiles must neither read nor write across batch members).
 bool self_check(talos_ctx* ctx) {
+  g_check_width = true;
   bool ok = self_check_shape(ctx, 200) && self_check_shape(ctx, 72, 88, 104, 3);
   g_check_fold = true;
   ok = ok && self_check_shape(ctx, 200, 328, 520);                               // K = 520 in one item on the one-CTA kernel: two chains, folded on chip
   g_check_fold = false;
   g_check_pair = true;
   ok = ok && self_check_shape(ctx, 456) && self_check_shape(ctx, 456, 328, 520);   // K = 520: two chains, folded on chip in 3xTF32 mode
-  g_check_pair = false;
+  g_check_pair = g_check_width = false;
   return ok;
 }
 

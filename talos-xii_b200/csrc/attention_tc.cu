@@ -80,9 +80,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   }
   if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
-  talos_pdl();
   __syncthreads();
   tc_fence_after();
+  talos_pdl();                             // this CTA holds its tensor memory
   const uint32_t tmem_base = *tmem_slot;
   const int first = blockIdx.x, step = gridDim.x;
 

@@ -84,10 +84,13 @@ inline void talos_check_ctx(talos_ctx* ctx) {
   TALOS_CHECK_CUDA(cudaSetDevice(ctx->device));
 }
 
-// Programmatic dependent launch.  Every kernel of the library starts with talos_pdl(): its CTAs may be set up while the
-// kernel before it on the stream is still running (its launch, its CTAs' set-up and its code fetch then overlap that
-// kernel's tail), they touch no memory before griddepcontrol.wait has seen that kernel complete, and they let the next
-// kernel be set up in turn.  The launch itself is cheaper, too: 2.07 -> 1.55 us of host time each, and a chain of tiny
+// Programmatic dependent launch.  Every kernel of the library calls talos_pdl() before it touches memory: its CTAs may be
+// set up while the kernel before it on the stream is still running (its launch, its CTAs' set-up and its code fetch then
+// overlap that kernel's tail), they read and write nothing before griddepcontrol.wait has seen that kernel complete, and they
+// let the next kernel be set up in turn.  It is the first statement but in the tensor-memory kernels, which call it behind the
+// block barrier that publishes their allocation: the call of any one thread lets the next kernel start, and two waiting
+// kernels' CTAs must not compete for an SM's columns (the later one would hold them and wait for the earlier one to
+// complete, the earlier one would wait for the columns).  The launch itself is cheaper, too: 2.07 -> 1.55 us of host time each, and a chain of tiny
 // dependent kernels takes 1.6 us a link instead of 2.1 (B200, driver 580).
 // The kernel's pointers are passed through it because a load that the compiler knows to be read-only (__restrict__ const, __ldg,
 // __ldcs) may otherwise be moved above the wait; kernels that take their pointers in a struct use plain loads.

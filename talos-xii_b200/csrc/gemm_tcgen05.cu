@@ -91,9 +91,9 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tmap_a, const CU
   }
   if (warp == 1) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
   tc_fence_before();
-  talos_pdl();                             // barriers and tensor memory were set up beside the previous kernel's tail; from here on memory is read
   __syncthreads();
   tc_fence_after();
+  talos_pdl();                             // barriers and tensor memory were set up beside the previous kernel's tail; from here on memory is read
   const uint32_t tmem_base = *tmem_slot;
 
   const int tiles_mn = g.m_tiles * g.n_tiles;

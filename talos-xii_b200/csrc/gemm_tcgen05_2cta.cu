@@ -89,10 +89,10 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   }
   if (warp == 1) { tmem_alloc2(tmem_slot, TMEM_COLS); tmem_relinquish2(); }
   tc_fence_before();
-  talos_pdl();
   __syncthreads();
   cluster_sync();                                              // the peer's barriers exist before anything is signalled on them
   tc_fence_after();
+  talos_pdl();                                                 // both CTAs hold their tensor memory
   const uint32_t tmem_base = *tmem_slot;
 
   const int tiles_mn = g.m_tiles * g.n_tiles;                  // m_tiles counts 256-row tiles here

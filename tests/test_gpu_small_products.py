@@ -68,6 +68,15 @@ def test_linear_backward(talos, ctx, rows, fin, fout, act, parts):
             assert np.array_equal(got[:-1], b.ravel().astype(np.float32))
 
 
+@pytest.mark.parametrize("rows,act", [(64, "tanh"), (64, "none"), (5000, "silu")])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_linear_backward_of_nothing(talos, ctx, rows, act, mode):
+    # every result may be left out, also all of them
+    x, W, dy = dev(normal(5, (rows, 16))), dev(normal(6, (16, 24))), dev(normal(7, (rows, 24)))
+    talos.lib.talos_linear_bwd(ctx.handle, talos.ptr(x), talos.ptr(W), talos.ptr(dy), talos.ptr(dy), None, None, None, rows, 16, 24, talos.ACTS[act], mode, 0)
+    ctx.synchronize()
+
+
 @pytest.mark.needs_tensor_cores
 @pytest.mark.parametrize("mode", [1, 2])
 @pytest.mark.parametrize("M,N,K", [(200, 72, 40), (129, 33, 100), (1000, 36, 520), (64, 260, 64)])

@@ -19,11 +19,14 @@ struct talos_error : std::runtime_error {
 
 void talos_set_last_error(const std::string& msg);
 
+// (The runtime keeps a failed call's error for cudaGetLastError, too: taken here, or the next launch would report it again.)
 #define TALOS_CHECK_CUDA(expr)                                                                     \
   do {                                                                                             \
     cudaError_t e__ = (expr);                                                                      \
-    if (e__ != cudaSuccess)                                                                        \
+    if (e__ != cudaSuccess) {                                                                      \
+      (void)cudaGetLastError();                                                                    \
       throw talos_error(TALOS_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(e__));      \
+    }                                                                                              \
   } while (0)
 
 #define TALOS_REQUIRE(cond, code, msg)                                                             \

@@ -32,6 +32,16 @@ def _expect(talos, status, fn):
     assert e.value.status == status, (e.value.status, str(e.value))
 
 
+def test_a_refused_launch_is_reported_once(talos, ctx):
+    # 65 536 blocks along the grid's second axis: refused by the runtime, nothing runs.  The next call has no part in it.
+    import torch
+    x = torch.zeros(65536 * 32, device="cuda:0"); y = torch.zeros_like(x)
+    shape = np.array([65536 * 32, 1], dtype=np.int64)
+    _expect(talos, talos.ERR_CUDA, lambda: talos.lib.talos_transpose(ctx.handle, talos.ptr(x), talos.ptr(y), talos.ptr(shape), 2, 0, 1, 0))
+    talos.lib.talos_eltwise_binary(ctx.handle, talos.EW["add"], talos.ptr(x), talos.ptr(x), talos.ptr(y), 16)
+    ctx.synchronize()
+
+
 def test_device_error_word_surfaces_from_every_blocking_entry_point(talos, ctx):
     import torch
     x = torch.arange(8, dtype=torch.float32, device="cuda:0")

@@ -77,6 +77,25 @@ def test_linear_backward_of_nothing(talos, ctx, rows, act, mode):
     ctx.synchronize()
 
 
+@pytest.mark.parametrize("over", ["dW over W", "dW over dy", "dW over saved", "db over W"])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_linear_backward_over_its_inputs(talos, ctx, over, mode):
+    # results over inputs that the steps before them have already used (dZ is a copy here, dX comes before dW and db)
+    n = 200
+    x, W, saved, dy = normal(5, (n, n)), normal(6, (n, n)), np.tanh(normal(7, (n, n))), normal(8, (n, n))
+    saved = saved.astype(np.float32).astype(np.float64)
+    dz = dy * (1 - saved ** 2)
+    t = dict(x=dev(x), W=dev(W), saved=dev(saved), dy=dev(dy))
+    out = dict(dx=dev(np.zeros((n, n))), dW=dev(np.zeros((n, n))), db=dev(np.zeros(n)))
+    result, source = over.split(" over ")
+    out[result] = t[source]
+    p = {k: talos.ptr(v) for k, v in {**t, **out}.items()}
+    talos.lib.talos_linear_bwd(ctx.handle, talos.ptr(t["x"]), talos.ptr(t["W"]), talos.ptr(t["saved"]), talos.ptr(t["dy"]), p["dx"], p["dW"], p["db"], n, n, n,
+                               talos.ACTS["tanh"], mode, 0)
+    assert rel_err(out["dx"], dz @ W.T) <= 1e-5 and rel_err(out["dW"], x.T @ dz) <= 1e-5
+    assert np.abs(host(out["db"]).ravel()[:n] - dz.sum(0)).max() <= 1e-5 * np.sqrt(n) * 4
+
+
 @pytest.mark.needs_tensor_cores
 @pytest.mark.parametrize("mode", [1, 2])
 @pytest.mark.parametrize("M,N,K", [(200, 72, 40), (129, 33, 100), (1000, 36, 520), (64, 260, 64)])

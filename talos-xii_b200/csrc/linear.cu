@@ -68,7 +68,7 @@ TALOS_API talos_status talos_linear_bwd(talos_ctx* ctx, const float* x, const fl
   // 3xTF32 mode (ten launches before), 1 024 x 256 x 256 56 -> 19 us; beyond that dW's reduction is too long for one
   // cluster and the tensor cores are faster (2 048 x 256 x 256: 36 against 57, 4 096 x 256 x 256: 68 against 59).  The
   // one launch reads its inputs while it writes its results, so a result that overlaps an input keeps the separate steps, which
-  // follow one another: dZ (a copy where there is an activation), dX, dW, db.
+  // follow one another: dZ (a copy, where there is an activation, and db with it), dX, dW.
   auto over_input = [&](const float* out, int64_t n) {
     auto hits = [&](const float* p, int64_t m) { return out && p && p < out + n && out < p + m; };
     return hits(dy, rows * out_f) || hits(act ? saved : nullptr, rows * out_f) || hits(x, rows * in_f) || hits(W, in_f * out_f);

@@ -77,7 +77,7 @@ def test_linear_backward_of_nothing(talos, ctx, rows, act, mode):
     ctx.synchronize()
 
 
-@pytest.mark.parametrize("over", ["dW over W", "dW over dy", "dW over saved", "db over W"])
+@pytest.mark.parametrize("over", ["dW over W", "dW over dy", "dW over saved", "db over dy", "db over saved"])
 @pytest.mark.parametrize("mode", [0, 1])
 def test_linear_backward_over_its_inputs(talos, ctx, over, mode):
     # results over inputs that the steps before them have already used (dZ is a copy here, dX comes before dW and db)

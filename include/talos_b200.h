@@ -12,6 +12,9 @@
  * Threading: a talos_ctx is one device + one stream; calls on one ctx must not overlap in time.
  * Work is enqueued on the ctx stream; only *_host entry points and talos_ctx_synchronize block.
  *
+ * Results must not overlap inputs unless a declaration says that they may (elementwise operations may
+ * write over an input of the same index).
+ *
  * Each declaration cites the reference item it replaces (paths are relative to the reference
  * crate root).
  */
@@ -147,7 +150,8 @@ talos_status talos_gemm_batched(talos_ctx* ctx, int32_t opA, int32_t opB, int64_
                                 int32_t beta, int32_t mode);
 
 /* ---- Linear (src/nn.rs:12-142), weight [in,out] row-major, y = act(x.W + b) ---------------- */
-/* z_save (nullable) receives the pre-activation (needed by SILU backward). */
+/* z_save (nullable) receives the pre-activation (needed by SILU backward).  Where in_features == out_features <= 64,
+ * y or z_save may be x. */
 talos_status talos_linear_fwd(talos_ctx* ctx, const float* x, const float* W, const float* bias, float* y,
                               float* z_save, int64_t rows, int64_t in_features, int64_t out_features,
                               int32_t act, int32_t mode);

@@ -195,6 +195,19 @@ __device__ __forceinline__ float talos_epilogue_apply(const EpiArgs& e, float ac
   return v;
 }
 
+// Whether a product's result (or the pre-activation it saves) overlaps an operand.  Such a product is sound only while ONE tile
+// spans its columns, so that a CTA has read its rows of A before it writes them (y = act(x.W) with y over x, a square layer): it
+// keeps the widest tile of its route, and the dispatch rules that would hand it to narrower ones ask here first.
+inline bool talos_result_over_operand(int opA, int opB, int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, int64_t strideA, const float* B, int64_t ldb,
+                                      int64_t strideB, const float* C, int64_t ldc, int64_t strideC, int64_t batch, const EpiArgs& e) {
+  if (K == 0) return false;
+  auto extent = [&](int64_t rows, int64_t cols, int64_t ld, int64_t stride) { return (rows - 1) * ld + cols + (batch > 1 ? (batch - 1) * stride : 0); };
+  const int64_t na = opA == TALOS_OP_N ? extent(M, K, lda, strideA) : extent(K, M, lda, strideA);
+  const int64_t nb = opB == TALOS_OP_N ? extent(K, N, ldb, strideB) : extent(N, K, ldb, strideB);
+  auto hits = [&](const float* p, int64_t n) { return p && ((A < p + n && p < A + na) || (B < p + n && p < B + nb)); };
+  return hits(C, extent(M, N, ldc, strideC)) || hits(e.aux_out, extent(M, N, e.ld_aux_out, 0));
+}
+
 // Internal cross-file entry points.
 void talos_gemm_fp32_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K, const float* A,
                             int64_t lda, int64_t strideA, const float* B, int64_t ldb, int64_t strideB, float* C,

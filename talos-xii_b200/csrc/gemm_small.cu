@@ -321,7 +321,8 @@ void talos_gemm_small_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_
   // shared out, since those sums cost more than 64 products do (65 536 x 64 x 8: 18 -> 9.1 us, 8 192 x 256 x 16: 11.3 -> 7.4; within
   // one round the shared-out range stays ahead, 1 200 x 256 x 64: 5.4 against 8.6, and so do 32 x 32 tiles, 8 192 x 16 x 256: 9.7
   // against 11.3).
-  const int tile = small_tile(ctx, ceil_div(M, 16) * ceil_div(N, 16) * batch, ceil_div(M, 32) * ceil_div(N, 32) * batch);
+  const bool in_place = talos_result_over_operand(opA, opB, M, N, K, A, lda, strideA, B, ldb, strideB, C, ldc, strideC, batch, epi);
+  const int tile = in_place ? 64 : small_tile(ctx, ceil_div(M, 16) * ceil_div(N, 16) * batch, ceil_div(M, 32) * ceil_div(N, 32) * batch);
   const bool rounds = ceil_div(M, 64) * ceil_div(N, 64) * batch > ctx->sm_count;
   if (tile == 16) TALOS_SMALL(16, 16, 2, 16, 128) else if (tile == 32) TALOS_SMALL(32, 32, 4, 8, 128) else if (N <= 16) TALOS_SMALL(64, 16, 4, 4, 64)
   else if (K <= 64 && rounds) TALOS_SMALL(64, 64, 4, 1, 32) else TALOS_SMALL(64, 64, 8, 4, 64)

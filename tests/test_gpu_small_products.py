@@ -7,7 +7,7 @@ import ctypes
 import numpy as np
 import pytest
 
-from gpu_util import dev, host, normal, rel_err
+from gpu_util import TOL, dev, host, normal, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -94,6 +94,22 @@ def test_linear_backward_over_its_inputs(talos, ctx, over, mode):
                                talos.ACTS["tanh"], mode, 0)
     assert rel_err(out["dx"], dz @ W.T) <= 1e-5 and rel_err(out["dW"], x.T @ dz) <= 1e-5
     assert np.abs(host(out["db"]).ravel()[:n] - dz.sum(0)).max() <= 1e-5 * np.sqrt(n) * 4
+
+
+@pytest.mark.parametrize("rows,width,modes", [(1, 8, (0, 1, 2)), (70, 36, (0, 1, 2)), (300, 64, (0, 1, 2)), (20000, 64, (0, 1, 2)), (33, 5, (0, 1, 2)),
+                                              (500, 128, (0, 1, 2)), (4736, 256, (1, 2)), (9000, 252, (1, 2))])
+@pytest.mark.parametrize("what", ["y", "z_save"])
+def test_square_linear_in_place(talos, ctx, rows, width, modes, what):
+    # y (or z_save) over x: one tile has to span the columns (64 on the CUDA cores, 128 for many rows, 256 on the tensor cores)
+    import torch
+    x, W, b = normal(5, (rows, width)), normal(6, (width, width), 1.0 / np.sqrt(width)), normal(7, (width,), 0.1)
+    w, bias, other = dev(W), dev(b), torch.empty(rows, width, device="cuda:0")
+    z = x @ W + b
+    for mode in modes:
+        io = dev(x)
+        y, save = (io, other) if what == "y" else (other, io)
+        talos.lib.talos_linear_fwd(ctx.handle, talos.ptr(io), talos.ptr(w), talos.ptr(bias), talos.ptr(y), talos.ptr(save), rows, width, width, talos.ACTS["tanh"], mode)
+        assert rel_err(save, z) <= TOL[mode] and rel_err(y, np.tanh(z)) <= TOL[mode], mode
 
 
 @pytest.mark.needs_tensor_cores

@@ -138,17 +138,33 @@ void talos_attention_launch(talos_ctx* ctx, HeadView q1, HeadView q2, HeadView k
 bool talos_attention_tc_fused(talos_ctx* ctx, const float* q, const float* k, const float* v, float* out, float* probs, int64_t BH,
                               int64_t S, int64_t dqk, int64_t dv, float scale, int causal);
 
+// Per-head tensors of a call, `width` floats a head.  The one-launch kernels read all of a head before they write any of it, but
+// write it while other CTAs read theirs: a result may only coincide with an input head by head.
+struct AttnHeads { const float* p; int64_t width; };
+static bool heads_apart(int64_t BH, std::initializer_list<AttnHeads> results, std::initializer_list<AttnHeads> inputs) {
+  for (const AttnHeads& r : results)
+    for (const AttnHeads& i : inputs)
+      if (r.p && r.p < i.p + BH * i.width && i.p < r.p + BH * r.width && !(r.p == i.p && r.width == i.width)) return false;
+  return true;
+}
+
 bool talos_attention_short_takes(talos_ctx* ctx, int64_t BH, int64_t S, int64_t dqk, int64_t dv, int mode, std::initializer_list<const void*> heads);
 void talos_attention_short_fwd(talos_ctx* ctx, const float* q, const float* k, const float* v, float* out, float* probs, int64_t BH, int64_t S, int64_t dqk, int64_t dv,
                                float scale, int causal);
 void talos_attention_short_bwd(talos_ctx* ctx, const float* q, const float* k, const float* v, const float* probs, const float* dout, float* dq, float* dk, float* dv, int64_t BH,
                                int64_t S, int64_t dqk, int64_t dvd, float scale);
 
+static bool short_fwd_takes(talos_ctx* ctx, const float* q, const float* k, const float* v, const float* out, const float* probs, int64_t BH, int64_t S, int64_t dqk,
+                            int64_t dv, int mode) {
+  return !(talos_switches() & SW_ATTN_NO_FUSED) && talos_attention_short_takes(ctx, BH, S, dqk, dv, mode, {q, k, v, out}) &&
+         heads_apart(BH, {{out, S * dv}, {probs, S * S}}, {{q, S * dqk}, {k, S * dqk}, {v, S * dv}});
+}
+
 static bool attention_fwd_tc(talos_ctx* ctx, const float* q, const float* k, const float* v, float* out, float* probs,
                              int64_t BH, int64_t S, int64_t dqk, int64_t dv, float scale, int causal, int mode) {
   // fast mode, S <= 128: one fused kernel with the scores in tensor memory (attention_tc.cu)
   if (mode == TALOS_MODE_TF32 && talos_attention_tc_fused(ctx, q, k, v, out, probs, BH, S, dqk, dv, scale, causal)) return true;
-  if (!(talos_switches() & SW_ATTN_NO_FUSED) && talos_attention_short_takes(ctx, BH, S, dqk, dv, mode, {q, k, v, out})) {
+  if (short_fwd_takes(ctx, q, k, v, out, probs, BH, S, dqk, dv, mode)) {
     talos_attention_short_fwd(ctx, q, k, v, out, probs, BH, S, dqk, dv, scale, causal);
     return true;
   }
@@ -174,7 +190,7 @@ TALOS_API talos_status talos_attention_fwd(talos_ctx* ctx, const float* q, const
   if (BH == 0 || S == 0) return TALOS_OK;
   TALOS_REQUIRE(q && k && v && out, TALOS_ERR_ARG, "null pointer");
   if (mode != TALOS_MODE_FP32 && attention_fwd_tc(ctx, q, k, v, out, probs, BH, S, dqk, dv, scale, causal ? 1 : 0, mode)) return TALOS_OK;
-  if (mode == TALOS_MODE_FP32 && !(talos_switches() & SW_ATTN_NO_FUSED) && talos_attention_short_takes(ctx, BH, S, dqk, dv, mode, {q, k, v, out})) {
+  if (mode == TALOS_MODE_FP32 && short_fwd_takes(ctx, q, k, v, out, probs, BH, S, dqk, dv, mode)) {
     talos_attention_short_fwd(ctx, q, k, v, out, probs, BH, S, dqk, dv, scale, causal ? 1 : 0);
     return TALOS_OK;
   }
@@ -198,7 +214,8 @@ TALOS_API talos_status talos_attention_bwd(talos_ctx* ctx, const float* q, const
   TALOS_REQUIRE(mode >= TALOS_MODE_FP32 && mode <= TALOS_MODE_TF32, TALOS_ERR_ARG, "bad arithmetic mode");
   if (BH == 0 || S == 0) return TALOS_OK;
   TALOS_REQUIRE(q && k && v && probs && dout && dq && dk && dv, TALOS_ERR_ARG, "null pointer");
-  if (!(talos_switches() & SW_ATTN_NO_FUSED) && talos_attention_short_takes(ctx, BH, S, dqk, dvd, mode, {q, k, v, dout, dq, dk, dv})) {
+  if (!(talos_switches() & SW_ATTN_NO_FUSED) && talos_attention_short_takes(ctx, BH, S, dqk, dvd, mode, {q, k, v, dout, dq, dk, dv}) &&
+      heads_apart(BH, {{dq, S * dqk}, {dk, S * dqk}, {dv, S * dvd}}, {{q, S * dqk}, {k, S * dqk}, {v, S * dvd}, {probs, S * S}, {dout, S * dvd}})) {
     talos_attention_short_bwd(ctx, q, k, v, probs, dout, dq, dk, dv, BH, S, dqk, dvd, scale);
     return TALOS_OK;
   }

@@ -59,3 +59,32 @@ def test_forward_and_backward(talos, S, dqk, dv, causal, mode, BH, offset):
             assert rel_err(got[:r.size], r.ravel()) <= tol, (n, rel_err(got[:r.size], r.ravel()))
         assert np.all(got[r.size:] == 7.0), n
     assert rel_err(host(bare[0])[offset:offset + ref["out"].size], ref["out"].ravel()) <= TOL[mode]
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("dqk,dv,result,source", [(16, 16, "out", "q"), (16, 16, "out", "v"), (16, 16, "dk", "q"), (16, 16, "dv", "do"), (32, 16, "out", "q"), (16, 32, "dk", "v")])
+def test_results_over_inputs(talos, mode, dqk, dv, result, source):
+    # Head by head in place: the one-launch kernels.  At another width heads meet each other's: the separate products, whose order
+    # allows it (fp32 mode has no such forward: its fused kernel, too, is one CTA a head).
+    if mode == 0 and dqk != dv and result == "out":
+        pytest.skip("heads of other widths over each other: tensor-core modes only")
+    BH, S, scale = 300, 48, 0.3
+    ctx, P, L = talos.torch_context(0), talos.ptr, talos.lib
+    a = dict(q=normal(1, (BH, S, dqk)), k=normal(2, (BH, S, dqk)), v=normal(3, (BH, S, dv)), do=normal(4, (BH, S, dv)))
+    s = (a["q"] @ a["k"].transpose(0, 2, 1)) * scale
+    p = np.exp(s - s.max(-1, keepdims=True)); p /= p.sum(-1, keepdims=True)
+    dp = a["do"] @ a["v"].transpose(0, 2, 1)
+    ds = scale * p * (dp - (dp * p).sum(-1, keepdims=True))
+    ref = dict(out=p @ a["v"], dk=ds.transpose(0, 2, 1) @ a["q"], dv=p.transpose(0, 2, 1) @ a["do"], dq=ds @ a["k"])
+    t = {n: dev(x) for n, x in a.items()}
+    t.update({n: dev(np.zeros(r.shape)) for n, r in ref.items()}, probs=dev(p))
+    t[result] = t[source]
+    held, t = t, {n: P(x) for n, x in t.items()}
+    if result == "out":
+        L.talos_attention_fwd(ctx.handle, t["q"], t["k"], t["v"], t["out"], None, BH, S, dqk, dv, scale, 0, mode)
+    else:
+        L.talos_attention_bwd(ctx.handle, t["q"], t["k"], t["v"], t["probs"], t["do"], t["dq"], t["dk"], t["dv"], BH, S, dqk, dv, scale, mode)
+    ctx.synchronize()
+    assert rel_err(host(held[result]).ravel()[:ref[result].size], ref[result].ravel()) <= TOL[mode]
+    if result != "out":
+        assert rel_err(held["dq"], ref["dq"]) <= TOL[mode]

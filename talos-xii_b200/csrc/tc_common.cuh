@@ -322,8 +322,9 @@ if (fuse && c < groups) {                                                       
         const bool straight = g.splits == 1 && groups == 8 && !dact && !g.epi.beta && (g.epi.act || g.epi.bias);
 #define TALOS_EPI_STRAIGHT(A, HAS_BIAS)                                                                                 \
   { const float4* bp = (const float4*)(g.epi.bias + n0);                                                                \
+    asm volatile("" : "+l"(bp));                                                                                        \
     _Pragma("unroll") for (int c = 0; c < 8; ++c) {                                                                    \
-      const float4 b4 = HAS_BIAS ? bp[c] : make_float4(0.f, 0.f, 0.f, 0.f);                                     \
+      const float4 b4 = HAS_BIAS ? __ldg(bp + c) : make_float4(0.f, 0.f, 0.f, 0.f);                              \
       r[4 * c] = __float_as_uint(talos_act(__uint_as_float(r[4 * c]) + b4.x, A));                                       \
       r[4 * c + 1] = __float_as_uint(talos_act(__uint_as_float(r[4 * c + 1]) + b4.y, A));                               \
       r[4 * c + 2] = __float_as_uint(talos_act(__uint_as_float(r[4 * c + 2]) + b4.z, A));                               \

@@ -10,7 +10,14 @@
 // the result is reproducible).
 #include "common.cuh"
 
+void talos_splitk_reduce(talos_ctx* ctx, const float* partial, int splits, int64_t M, int64_t N, float* C, int64_t ldc, const EpiArgs& epi);
+
 namespace {
+
+// Reductions longer than this for each CTA of an unslabbed product are cut into slabs.  fp32 mode, x^T.dZ: 64 x 64 x 65 536
+// 104 -> 35 us, 64 x 16 x 65 536 60 -> 20, 16 x 16 x 1 048 576 936 -> 75, 256 x 32 x 65 536 106 -> 56, 64 x 256 x 8 192 29 -> 21; at
+// 1 024 it is even or slower (64 x 256 x 4 096 16.5 -> 19.1, 64 x 512 x 2 048 18.7 -> 20.6).
+constexpr int64_t SLAB_WALK = 1024;
 
 struct SmallOperand {
   const float* p; long long ld, batch;      // element (r, k): p[r*ld + k] when k_contig, else p[k*ld + r]
@@ -21,6 +28,7 @@ struct SmallProduct {
   SmallOperand a, b;
   float* C; long long ldc, batchC; int vec_c;
   int M, N, K, m_tiles, n_tiles, batch, splits, k_split;    // splits: a power of two; k_split: reduction elements per split, whole chunks
+  int k_slab;                               // > 0: batch member z reduces k_slab elements from z * k_slab on (a long reduction in slabs)
   float* colsum; int colsum_acc;            // column sums of B over the whole reduction (the bias gradient), by the m_tile 0 CTAs
   EpiArgs epi;
 };
@@ -142,7 +150,8 @@ __device__ __forceinline__ void small_product(const SmallProduct& g, unsigned it
     if (g.splits > 1) { cluster_barrier(); cluster_barrier(); }
     return;
   }
-  const int m0 = mt * BM, n0 = nt * BN, k_begin = min(g.K, (int)split * g.k_split), k_end = min(g.K, k_begin + g.k_split);
+  const int m0 = mt * BM, n0 = nt * BN, k_first = (int)bz * g.k_slab, k_last = g.k_slab ? min(g.K, k_first + g.k_slab) : g.K;
+  const int k_begin = min(k_last, k_first + (int)split * g.k_split), k_end = min(k_last, k_begin + g.k_split);
   const long long base_a = bz * g.a.batch, base_b = bz * g.b.batch;
   const bool want_sum = DACT && g.colsum && mt == 0;
   SmallTile<BM, KC, T, LA, VEC, DACT> ta; SmallTile<BN, KC, T, LB, VEC, DACT> tb;
@@ -262,6 +271,7 @@ linear_bwd_small_kernel(const __grid_constant__ SmallProduct gx, const __grid_co
   small_product<BM, BN, TM, KG, KC, VEC, true>(w_role ? gw : gx, w_role ? blockIdx.x : blockIdx.x - items_w, sm);
 }
 
+int64_t small_tiles(int64_t M, int64_t N, int bm, int bn) { return ceil_div(M, bm) * ceil_div(N, bn); }
 bool small_vec(const SmallOperand& o, int64_t rows, int64_t K) {
   return (((uintptr_t)o.p | (uintptr_t)(o.dact ? o.saved : nullptr)) & 15) == 0 && !(o.ld & 3) && !(o.batch & 3) && !((o.k_contig ? K : rows) & 3);
 }
@@ -269,7 +279,7 @@ bool small_vec(const SmallOperand& o, int64_t rows, int64_t K) {
 // eight of a portable cluster (adding up the partial tiles takes about as long as one chunk).
 void small_shape(talos_ctx* ctx, SmallProduct& g, int bm, int bn, int kc, int64_t batch, int64_t slots) {
   g.m_tiles = (int)ceil_div(g.M, bm); g.n_tiles = (int)ceil_div(g.N, bn); g.batch = (int)batch;
-  const int64_t tiles = (int64_t)g.m_tiles * g.n_tiles * batch, chunks = std::max<int64_t>(1, ceil_div(g.K, kc));
+  const int64_t tiles = (int64_t)g.m_tiles * g.n_tiles * batch, chunks = std::max<int64_t>(1, ceil_div(g.k_slab ? g.k_slab : g.K, kc));
   int splits = 1;
   while (splits < 8 && splits < chunks && tiles * splits * 2 <= slots) splits *= 2;
   g.splits = splits; g.k_split = (int)(ceil_div(chunks, splits) * kc);
@@ -301,7 +311,26 @@ void launch_bwd(talos_ctx* ctx, SmallProduct& gx, SmallProduct& gw, int64_t slot
                        (unsigned)items_w);
 }
 
+// Tile of a product with a long reduction and few tiles: the widest that its result fills, since operands are re-read once
+// per tile across them and the slabs keep the SMs busy anyway.
+struct SlabTile { int bm, bn, ctas; };
+SlabTile slab_tile(int64_t M, int64_t N) {
+  if (M > 32 && N > 32) return {64, 64, SmallCfg<64, 64, 4, 1, 32>::CTAS};
+  if (M > 16 && N <= 16) return {64, 16, SmallCfg<64, 16, 4, 4, 64>::CTAS};
+  if (M > 16) return {32, 32, SmallCfg<32, 32, 4, 8, 128>::CTAS};
+  return {16, 16, SmallCfg<16, 16, 2, 16, 128>::CTAS};
+}
+
 }  // namespace
+
+// Reduction elements one CTA walks for a plain product on these kernels.
+int64_t talos_gemm_small_walk(talos_ctx* ctx, int64_t M, int64_t N, int64_t K) {
+  const int tile = small_tile(ctx, small_tiles(M, N, 16, 16), small_tiles(M, N, 32, 32));
+  const int64_t tiles = small_tiles(M, N, tile, tile), slots = (tile == 64 ? 1 : 2) * (int64_t)ctx->sm_count, chunks = ceil_div(K, tile == 64 ? 64 : 128);
+  int64_t splits = 1;
+  while (splits < 8 && splits < chunks && tiles * splits * 2 <= slots) splits *= 2;
+  return ceil_div(K, splits);
+}
 
 // C = op(A).op(B) with the epilogue, any shape and alignment.
 void talos_gemm_small_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, int64_t strideA, const float* B,
@@ -316,6 +345,25 @@ void talos_gemm_small_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_
   // take 1 024 cycles for a chunk of a 32 x 32 tile and a quarter of that for a 16 x 16 one, which is what is left once
   // the launch and the loads are as short as they get; larger tiles re-read the operands less often.
 #define TALOS_SMALL(BM, BN, TM, KG, KC) { if (vec) launch_gemm<BM, BN, TM, KG, KC, true>(ctx, g, batch); else launch_gemm<BM, BN, TM, KG, KC, false>(ctx, g, batch); }
+  // Few tiles and a long reduction (a first layer's weight gradient over a large fp32 minibatch): a cluster's eight CTAs would
+  // walk it alone, so it is cut into slabs, a cluster each, as many as fill the SMs; their results go through memory.
+  if (batch == 1 && talos_gemm_small_walk(ctx, M, N, K) > SLAB_WALK) {
+    const SlabTile t = slab_tile(M, N);
+    const int64_t tiles = small_tiles(M, N, t.bm, t.bn), slots = t.ctas * (int64_t)ctx->sm_count;
+    int64_t cluster = 8;          // narrower clusters, more slabs, where eight to a cluster would leave more than a thirtieth of the slots empty
+    while (cluster > 1 && slots / (tiles * cluster) * tiles * cluster * 30 < slots * 29) cluster /= 2;
+    const int64_t want = std::min(slots / (tiles * cluster), K / 1024);
+    if (want > 1) {
+      g.k_slab = (int)(ceil_div(ceil_div(K, want), 128) * 128);       // whole chunks: the vector loads stay aligned
+      batch = ceil_div(K, g.k_slab);
+      g.C = (float*)talos_workspace(ctx, sizeof(float) * (size_t)(batch * M * N)); g.ldc = N; g.batchC = M * N; g.vec_c = !(N & 3); g.epi = EpiArgs{};
+      if (t.bm == 16) TALOS_SMALL(16, 16, 2, 16, 128) else if (t.bm == 32) TALOS_SMALL(32, 32, 4, 8, 128) else if (t.bn == 16) TALOS_SMALL(64, 16, 4, 4, 64)
+      else TALOS_SMALL(64, 64, 4, 1, 32)
+      talos_launched(ctx, "gemm_small");
+      talos_splitk_reduce(ctx, g.C, (int)batch, M, N, C, ldc, epi);
+      return;
+    }
+  }
   // Past one round, three CTAs of 256 threads an SM hide each other's loads and stores: a narrow result (a head's logits) takes
   // 64 x 16 tiles (65 536 x 5 x 64: 31 -> 13 us, 20 000 x 5 x 64: 13.5 -> 5.9), a short reduction tiles whose k range is not
   // shared out, since those sums cost more than 64 products do (65 536 x 64 x 8: 18 -> 9.1 us, 8 192 x 256 x 16: 11.3 -> 7.4; within

@@ -35,6 +35,27 @@ def test_product(talos, ctx, M, N, K, opA, opB):
     assert np.all(got[M] == -7.0)                                # nothing past the last row
 
 
+@pytest.mark.parametrize("M,N,K", [(64, 64, 9001), (64, 64, 65536), (33, 5, 20000), (8, 64, 9000), (16, 16, 40004), (70, 20, 33335), (40, 36, 16384), (300, 12, 16387)])
+@pytest.mark.parametrize("opA,opB", [(1, 0), (0, 1)])
+def test_long_reduction(talos, ctx, M, N, K, opA, opB):
+    # slabs of the reduction whose results go through memory: ends inside a slab and a chunk, every tile of that route, the epilogue
+    # behind the sum.  Rounding: sums of K / (slabs * splits * groups) terms, then of those sums; 1e-5 is ten times that.
+    import torch
+    A, B = normal(1, (K, M) if opA else (M, K)), normal(2, (N, K) if opB else (K, N), 1.0 / np.sqrt(K))
+    bias, C0 = normal(3, (N,)), normal(4, (M, N))
+    a, b, bi, c = dev(A), dev(B), dev(bias), dev(np.pad(C0, ((0, 1), (0, 0)), constant_values=-7.0))
+    epi = talos.Epilogue(bias=talos.ptr(bi), act=talos.ACT_TANH, beta=1)
+    args = (ctx.handle, opA, opB, M, N, K, talos.ptr(a), A.shape[1], talos.ptr(b), B.shape[1])
+    talos.lib.talos_gemm(*args, talos.ptr(c), N, 0, ctypes.byref(epi))
+    ref = (A.T if opA else A) @ (B.T if opB else B)
+    got = host(c)
+    assert rel_err(got[:M], C0 + np.tanh(ref + bias)) <= 1e-5 and np.all(got[M] == -7.0)
+    plain = [torch.empty(M, N, device="cuda:0") for _ in range(2)]
+    for p in plain:
+        talos.lib.talos_gemm(*args, talos.ptr(p), N, 0, None)
+    assert rel_err(plain[0], ref) <= 1e-5 and torch.equal(plain[0], plain[1])
+
+
 @pytest.mark.parametrize("rows,fin,fout", [(1, 1, 1), (64, 8, 64), (64, 64, 1), (64, 64, 5), (129, 12, 20), (300, 64, 64), (1100, 7, 33), (4096, 8, 16), (500, 256, 256)])
 @pytest.mark.parametrize("act", ["none", "tanh", "relu", "silu"])
 @pytest.mark.parametrize("parts", ["all", "dx", "dw", "accumulate"])

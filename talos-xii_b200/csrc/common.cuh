@@ -214,7 +214,9 @@ void talos_gemm_fp32_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t
                             int64_t ldc, int64_t strideC, int64_t batch, const EpiArgs& epi);
 void talos_gemm_small_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, int64_t strideA, const float* B,
                              int64_t ldb, int64_t strideB, float* C, int64_t ldc, int64_t strideC, int64_t batch, const EpiArgs& epi);
-void talos_linear_bwd_small_launch(talos_ctx* ctx, const float* x, const float* W, const float* saved, const float* dy, float* dx, float* dW, float* db,
+// Reduction elements that one CTA of these kernels walks for a plain product.
+int64_t talos_gemm_small_walk(talos_ctx* ctx, int64_t M, int64_t N, int64_t K);
+bool talos_linear_bwd_small_launch(talos_ctx* ctx, const float* x, const float* W, const float* saved, const float* dy, float* dx, float* dW, float* db,
                                    int64_t rows, int64_t in_f, int64_t out_f, int act, int accumulate);
 // Returns false when the shape/alignment is not eligible (caller falls back to the fp32 kernel).
 // First stage of the column sums only: dZ = dY * act'(saved) when dact != 0 (dz may alias dy) and the per-slab column

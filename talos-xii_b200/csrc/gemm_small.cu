@@ -296,13 +296,24 @@ void launch_gemm(talos_ctx* ctx, SmallProduct& g, int64_t batch) {
 template <int BM, int TM, int KG, int KC, bool VEC>
 void launch_bwd(talos_ctx* ctx, SmallProduct& gx, SmallProduct& gw, int64_t slots) {
   using Cfg = SmallCfg<BM, BM, TM, KG, KC>;
-  int64_t items_w = 0, items_x = 0;
-  gx.splits = gw.splits = 1;
-  if (gw.C) {       // the longer reduction: it gets what dX's tiles leave
-    const int64_t tiles_x = gx.C ? ceil_div(gx.M, BM) * ceil_div(gx.N, BM) : 0;
-    small_shape(ctx, gw, BM, BM, KC, 1, std::max(slots - tiles_x, slots / 2)); items_w = (int64_t)gw.m_tiles * gw.n_tiles * gw.splits;
-  }
-  if (gx.C) { small_shape(ctx, gx, BM, BM, KC, 1, slots - items_w); items_x = (int64_t)gx.m_tiles * gx.n_tiles * gx.splits; }
+  // How far either reduction is split: the pair that is over first.  A CTA takes its chunks, about two more for its start and its
+  // stores and half a one for each doubling of the partial tiles that are added up; past one round of CTAs their work
+  // counts, too.  (Leaving dX what dW's split does not take gave dX none: 128 x 512 x 512 28.7 -> 10.9 us.)
+  const int64_t tiles_w = gw.C ? small_tiles(gw.M, gw.N, BM, BM) : 0, tiles_x = gx.C ? small_tiles(gx.M, gx.N, BM, BM) : 0;
+  const int64_t chunks_w = ceil_div(gw.K, KC), chunks_x = ceil_div(gx.K, KC);
+  double best = -1.0;
+  for (int sw = 1; sw <= (gw.C ? 8 : 1) && (sw == 1 || sw / 2 < chunks_w); sw *= 2)
+    for (int sx = 1; sx <= (gx.C ? 8 : 1) && (sx == 1 || sx / 2 < chunks_x); sx *= 2) {
+      const auto taken = [](int64_t chunks, int s) { return (double)ceil_div(chunks, s) + 2.0 + (s == 1 ? 0.0 : s == 2 ? 0.5 : s == 4 ? 1.0 : 1.5); };
+      const double cw = tiles_w ? taken(chunks_w, sw) : 0.0, cx = tiles_x ? taken(chunks_x, sx) : 0.0;
+      const double cost = std::max(cw, cx) + (tiles_w * sw + tiles_x * sx > slots ? (tiles_w * sw * cw + tiles_x * sx * cx) / (double)slots : 0.0);
+      if (best < 0.0 || cost < best) { best = cost; gw.splits = sw; gx.splits = sx; }
+    }
+  auto shape = [&](SmallProduct& g, int64_t chunks) {
+    g.m_tiles = (int)ceil_div(g.M, BM); g.n_tiles = (int)ceil_div(g.N, BM); g.batch = 1; g.k_split = (int)(ceil_div(chunks, g.splits) * KC);
+  };
+  shape(gw, chunks_w); shape(gx, chunks_x);
+  int64_t items_w = tiles_w * gw.splits; const int64_t items_x = tiles_x * gx.splits;
   const int cluster = std::max(gx.splits, gw.splits);
   items_w = ceil_div(items_w, cluster) * cluster;
   static std::atomic<uint64_t> smem_set{0};
@@ -379,9 +390,13 @@ void talos_gemm_small_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_
 }
 
 // dX (+)= dZ.W^T, dW (+)= x^T.dZ, db (+)= column sums of dZ, dZ = dY * act'(saved), in one launch (dx or dW/db may be null;
-// db comes with dW).
-void talos_linear_bwd_small_launch(talos_ctx* ctx, const float* x, const float* W, const float* saved, const float* dy, float* dx, float* dW, float* db,
+// db comes with dW).  False, nothing launched: dW alone has more tiles than a round of CTAs.
+bool talos_linear_bwd_small_launch(talos_ctx* ctx, const float* x, const float* W, const float* saved, const float* dy, float* dx, float* dW, float* db,
                                    int64_t rows, int64_t in_f, int64_t out_f, int act, int accumulate) {
+  const int tile = small_tile(ctx, (dx ? small_tiles(rows, in_f, 16, 16) : 0) + (dW ? small_tiles(in_f, out_f, 16, 16) : 0),
+                              (dx ? small_tiles(rows, in_f, 32, 32) : 0) + (dW ? small_tiles(in_f, out_f, 32, 32) : 0));
+  const int64_t slots = (tile == 64 ? 1 : 2) * (int64_t)ctx->sm_count;
+  if (dW && small_tiles(in_f, out_f, tile, tile) > slots) return false;
   SmallProduct gx{}, gw{};
   bool vec = true;
   if (dx) {
@@ -397,10 +412,8 @@ void talos_linear_bwd_small_launch(talos_ctx* ctx, const float* x, const float* 
     vec = vec && small_vec(gw.a, in_f, rows) && small_vec(gw.b, out_f, rows);
   }
 #define TALOS_SMALL(BM, TM, KG, KC) { if (vec) launch_bwd<BM, TM, KG, KC, true>(ctx, gx, gw, slots); else launch_bwd<BM, TM, KG, KC, false>(ctx, gx, gw, slots); }
-  const int tile = small_tile(ctx, (dx ? ceil_div(rows, 16) * ceil_div(in_f, 16) : 0) + (dW ? ceil_div(in_f, 16) * ceil_div(out_f, 16) : 0),
-                              (dx ? ceil_div(rows, 32) * ceil_div(in_f, 32) : 0) + (dW ? ceil_div(in_f, 32) * ceil_div(out_f, 32) : 0));
-  const int64_t slots = (tile == 64 ? 1 : 2) * (int64_t)ctx->sm_count;
   if (tile == 16) TALOS_SMALL(16, 2, 16, 128) else if (tile == 32) TALOS_SMALL(32, 4, 8, 128) else TALOS_SMALL(64, 8, 4, 64)
 #undef TALOS_SMALL
   talos_launched(ctx, "linear_bwd_small");
+  return true;
 }

@@ -66,7 +66,9 @@ TALOS_API talos_status talos_linear_bwd(talos_ctx* ctx, const float* x, const fl
   if (!dx && !dW && !db) return TALOS_OK;
   // Up to 4 096 rows and 2^26 products everything runs as one launch on the CUDA cores: 512 x 64 x 64 with tanh 38 -> 6.5 us in
   // 3xTF32 mode (ten launches before), 1 024 x 256 x 256 56 -> 19 us; beyond that dW's reduction is too long for one
-  // cluster and the tensor cores are faster (2 048 x 256 x 256: 36 against 57, 4 096 x 256 x 256: 68 against 59).  The
+  // cluster and the tensor cores are faster (2 048 x 256 x 256: 36 against 57, 4 096 x 256 x 256: 68 against 59).  A wide layer
+  // of few rows, whose dW has more tiles than a round of CTAs, also keeps the separate products: its blocks would be all
+  // prologue and store (16 x 2 048 x 2 048 112 us in one launch against 35, 8 x 1 024 x 4 096 200 / 32, 64 x 1 024 x 1 024 59 / 39).  The
   // one launch reads its inputs while it writes its results, so a result that overlaps an input keeps the separate steps, which
   // follow one another: dZ (a copy, where there is an activation, and db with it), dX, dW.
   auto over_input = [&](const float* out, int64_t n) {
@@ -74,10 +76,9 @@ TALOS_API talos_status talos_linear_bwd(talos_ctx* ctx, const float* x, const fl
     return hits(dy, rows * out_f) || hits(act ? saved : nullptr, rows * out_f) || hits(x, rows * in_f) || hits(W, in_f * out_f);
   };
   if (rows <= 4096 && rows * in_f * out_f <= (1LL << 26) && (dW || !db) && !(talos_switches() & SW_TC_NO_SMALL) && !over_input(dx, rows * in_f) &&
-      !over_input(dW, in_f * out_f) && !over_input(db, out_f)) {
-    talos_linear_bwd_small_launch(ctx, x, W, saved, dy, dx, dW, db, rows, in_f, out_f, act, accumulate);
+      !over_input(dW, in_f * out_f) && !over_input(db, out_f) &&
+      talos_linear_bwd_small_launch(ctx, x, W, saved, dy, dx, dW, db, rows, in_f, out_f, act, accumulate))
     return TALOS_OK;
-  }
   const float* dz = dy;
   bool db_done = false;
   if (act != TALOS_ACT_NONE) {

@@ -56,7 +56,7 @@ def test_long_reduction(talos, ctx, M, N, K, opA, opB):
     assert rel_err(plain[0], ref) <= 1e-5 and torch.equal(plain[0], plain[1])
 
 
-@pytest.mark.parametrize("rows,fin,fout", [(1, 1, 1), (64, 8, 64), (64, 64, 1), (64, 64, 5), (129, 12, 20), (300, 64, 64), (1100, 7, 33), (4096, 8, 16), (500, 256, 256)])
+@pytest.mark.parametrize("rows,fin,fout", [(128, 512, 512), (64, 256, 1024), (2048, 40, 300), (1, 1, 1), (64, 8, 64), (64, 64, 1), (64, 64, 5), (129, 12, 20), (300, 64, 64), (1100, 7, 33), (4096, 8, 16), (500, 256, 256)])
 @pytest.mark.parametrize("act", ["none", "tanh", "relu", "silu"])
 @pytest.mark.parametrize("parts", ["all", "dx", "dw", "accumulate"])
 def test_linear_backward(talos, ctx, rows, fin, fout, act, parts):

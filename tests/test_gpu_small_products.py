@@ -56,6 +56,21 @@ def test_long_reduction(talos, ctx, M, N, K, opA, opB):
     assert rel_err(plain[0], ref) <= 1e-5 and torch.equal(plain[0], plain[1])
 
 
+@pytest.mark.parametrize("rows,fin,fout", [(1, 4100, 4096), (16, 2048, 2048), (3, 700, 3000)])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_wide_layer_of_few_rows(talos, ctx, rows, fin, fout, mode):
+    # on either side of where a product of few rows is walked too long for these kernels, and dW has more tiles than a round of blocks
+    import torch
+    x, W, dy = normal(5, (rows, fin)), normal(6, (fin, fout), 0.02), normal(8, (rows, fout))
+    tx, tw, ty = dev(x), dev(W), dev(dy)
+    y, dx, dW, db = (torch.empty(*s, device="cuda:0") for s in ((rows, fout), (rows, fin), (fin, fout), (fout,)))
+    P = talos.ptr
+    talos.lib.talos_linear_fwd(ctx.handle, P(tx), P(tw), None, P(y), None, rows, fin, fout, 0, mode)
+    talos.lib.talos_linear_bwd(ctx.handle, P(tx), P(tw), None, P(ty), P(dx), P(dW), P(db), rows, fin, fout, 0, mode, 0)
+    for got, ref in ((y, x @ W), (dx, dy @ W.T), (dW, x.T @ dy), (db, dy.sum(0))):
+        assert rel_err(got, ref) <= TOL[mode]
+
+
 @pytest.mark.parametrize("rows,fin,fout", [(128, 512, 512), (64, 256, 1024), (2048, 40, 300), (1, 1, 1), (64, 8, 64), (64, 64, 1), (64, 64, 5), (129, 12, 20), (300, 64, 64), (1100, 7, 33), (4096, 8, 16), (500, 256, 256)])
 @pytest.mark.parametrize("act", ["none", "tanh", "relu", "silu"])
 @pytest.mark.parametrize("parts", ["all", "dx", "dw", "accumulate"])

@@ -186,8 +186,10 @@ void talos_gemm_fp32_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t
                             int64_t lda, int64_t strideA, const float* B, int64_t ldb, int64_t strideB, float* C,
                             int64_t ldc, int64_t strideC, int64_t batch, const EpiArgs& epi) {
   // The 128 x 128 kernel takes products that give at least half of the SMs a tile, or whose long reduction it can split to do
-  // so (the weight-gradient shape: M, N <= 256 with K = the minibatch); everything smaller goes to the small kernel, and so
-  // do short reductions, where this one is all scattered epilogue (8 192 x 256 x 16: 28 against 8 us).
+  // so (the weight gradient of two wide layers, 96 <= M, N, with K = the minibatch); everything smaller or narrower goes to the
+  // small kernels, and so do short reductions, where this one spends its time in its scattered epilogue, whatever M and N
+  // (this kernel against those: 8 192 x 256 x 16 28 against 8 us, 65 536 x 256 x 64 273 / 88, 65 536 x 1 024 x 128 1 426 / 773,
+  // 4 096 x 4 096 x 128 352 / 196, 2 048 x 2 048 x 200 127 / 69, 1 024 x 1 024 x 200 62 / 21).
   const int64_t tiles = ceil_div(M, 128) * ceil_div(N, 128) * batch;
   int splits = 1;
   if (batch == 1 && tiles * 2 <= ctx->sm_count && K >= 2048) {

@@ -154,15 +154,18 @@ void small_steps(talos_ppo* p, const float* obs, const int32_t* actions, const f
   p->t += steps; p->steps_in_epoch += steps; p->weights_prepared = false; p->last_launches = 1;
 }
 
+// A small policy comes here for the steps that exchange gradients.  Its log-probabilities are the one-launch forward's, fp32 in
+// every mode; the step's own have to be, too, or the first ratio of an update would differ from 1 by TF32 rounding.
 void forward(talos_ppo* p, const float* obs, int64_t n) {
   const auto& c = p->cfg; const float* P = p->params;
   ensure_weights_prepared(p);
-  EpiArgs e1{P + p->o_b1, nullptr, 0, nullptr, 0, TALOS_ACT_TANH, 0, 0};
-  gemm_w(p, 0, 0, n, c.hidden, c.obs_dim, obs, c.obs_dim, p->o_w1, c.hidden, p->h1, c.hidden, e1);
-  EpiArgs e2{P + p->o_b2, nullptr, 0, nullptr, 0, TALOS_ACT_TANH, 0, 0};
-  gemm_w(p, 0, 0, n, c.hidden, c.hidden, p->h1, c.hidden, p->o_w2, c.hidden, p->h2, c.hidden, e2);
-  EpiArgs e3{P + p->o_bh, nullptr, 0, nullptr, 0, 0, 0, 0};
-  gemm_w(p, 0, 0, n, p->HP, c.hidden, p->h2, c.hidden, p->o_wh, p->HP, p->z, p->HP, e3);
+  auto product = [&](int64_t N, int64_t K, const float* A, int64_t w_off, float* C, const EpiArgs& e) {
+    if (p->small_cluster) talos_gemm_fp32_launch(p->ctx, 0, 0, n, N, K, A, K, 0, P + w_off, N, 0, C, N, 0, 1, e);
+    else gemm_w(p, 0, 0, n, N, K, A, K, w_off, N, C, N, e);
+  };
+  product(c.hidden, c.obs_dim, obs, p->o_w1, p->h1, EpiArgs{P + p->o_b1, nullptr, 0, nullptr, 0, TALOS_ACT_TANH, 0, 0});
+  product(c.hidden, c.hidden, p->h1, p->o_w2, p->h2, EpiArgs{P + p->o_b2, nullptr, 0, nullptr, 0, TALOS_ACT_TANH, 0, 0});
+  product(p->HP, c.hidden, p->h2, p->o_wh, p->z, EpiArgs{P + p->o_bh, nullptr, 0, nullptr, 0, 0, 0, 0});
 }
 
 void pack_params(talos_ppo* p, const float* canon, float* internal) {

@@ -73,3 +73,21 @@ def test_an_unknown_action_is_reported(talos, ctx):
         ctx.synchronize()
     ctx.synchronize()
     tr.close()
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_one_forward_with_and_without_a_communicator(talos, ctx, mode):
+    # The log-probabilities stored before an update and those of its first step, taken with a communicator (of one rank), come from
+    # the same arithmetic.  Logits of about 30: fp32 rounding puts 1e-5 into a log-ratio and 2^-24 into (ratio - 1) - log(ratio); TF32
+    # on one side would put 1e-2 into the log-ratio and 1e-4 into the KL.
+    import torch
+    n = 512
+    obs, actions, adv, ret, params = make_problem(n, 8, 64, 5, seed=230)
+    params["wp"] = orc.f32r(params["wp"] * 12.0)
+    comm = talos.Comm(ctx, talos.Comm.unique_id(), 1, 0)
+    tr = talos.PPOTrainer(ctx, talos.PpoConfig(8, 64, 5, n, mode), comm); tr.set_params(params)
+    d_obs, d_act, old = dev(obs), dev(actions), torch.empty(n, device="cuda")
+    tr.log_prob(d_obs, d_act, n, old)
+    kls = tr.update(d_obs, d_act, old, dev(adv), dev(ret), n, 1, 0.0)
+    assert abs(kls[0]) <= 1e-6, kls
+    tr.close(); comm.close()

@@ -360,10 +360,12 @@ void talos_gemm_small_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_
   // walk it alone, so it is cut into slabs, a cluster each, as many as fill the SMs; their results go through memory.
   if (batch == 1 && talos_gemm_small_walk(ctx, M, N, K) > SLAB_WALK) {
     const SlabTile t = slab_tile(M, N);
-    const int64_t tiles = small_tiles(M, N, t.bm, t.bn), slots = t.ctas * (int64_t)ctx->sm_count;
-    int64_t cluster = 8;          // narrower clusters, more slabs, where eight to a cluster would leave more than a thirtieth of the slots empty
-    while (cluster > 1 && slots / (tiles * cluster) * tiles * cluster * 30 < slots * 29) cluster /= 2;
-    const int64_t want = std::min(slots / (tiles * cluster), K / 1024);
+    // as many clusters as there are slots, or fewer where the SMs then share them more evenly
+    const int64_t tiles = small_tiles(M, N, t.bm, t.bn), sms = ctx->sm_count, most = t.ctas * sms / (8 * tiles);
+    auto filled = [&](int64_t slabs) { const int64_t ctas = 8 * tiles * slabs; return (double)ctas / (double)(ceil_div(ctas, sms) * sms); };
+    int64_t even = most;
+    for (int64_t s = most; s > 0 && 2 * s >= most; --s) if (filled(s) > filled(even) + 0.01) even = s;
+    const int64_t want = std::min(even, K / 1024);
     if (want > 1) {
       g.k_slab = (int)(ceil_div(ceil_div(K, want), 128) * 128);       // whole chunks: the vector loads stay aligned
       batch = ceil_div(K, g.k_slab);

@@ -795,12 +795,11 @@ bool talos_gemm_tc_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N
   // preparation + tiles that fill a few SMs: 11 to 25 us) and stay on the CUDA cores (gemm_small.cu: 512 x 64 x 64 11.3 -> 4.2 us,
   // 512 x 256 x 256 24.6 -> 10.3, 4 096 x 64 x 256 even) unless the caller brings prepared weights or a fused epilogue or the
   // reduction that a CTA would walk there is long: 30 x 1 448 x 1 448 22 us there, 20 here in 3xTF32 and 15 in TF32, 1 x 4 096 x
-  // 4 096 48 against 31 and 19; at 1 024 that route is ahead (1 x 2 048 x 2 048 15 against 20).  At 2^26 itself it still is in
-  // 3xTF32 (256 x 512 x 512 12 against 22, 64 x 1 024 x 1 024 18 / 24), not for short reductions (4 096 x 256 x 64 11 / 9).
+  // 4 096 48 against 31 and 19; at 1 024 that route is ahead (1 x 2 048 x 2 048 15 against 20).
   if ((((uintptr_t)A | (uintptr_t)B) & 15) || (lda & 3) || (ldb & 3) || K < 1) return false;
   const bool small_ok = !extra && K <= 4096 && !(talos_switches() & SW_TC_NO_SMALL) && talos_gemm_small_walk(ctx, M, N, K) <= 1024 &&
                         !talos_result_over_operand(opA, opB, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, epi);
-  if (M * N * K < (small_ok ? (1LL << 26) + (x3_mode(mode) && K >= 128 ? 1 : 0) : 1LL << 18) || M < 1 || N < 1) return false;
+  if (M * N * K < (small_ok ? 1LL << 26 : 1LL << 18) || M < 1 || N < 1) return false;
   if (!tc_ready(ctx)) return false;
   if (extra && extra->b_hi && ((((uintptr_t)extra->b_hi | (uintptr_t)extra->b_lo) & 15) != 0)) return false;
   tc_launch(ctx, opA, opB, M, N, K, A, lda, B, ldb, C, ldc, mode, epi, TcBatch{1, 0, 0, 0}, extra);

@@ -75,10 +75,13 @@ TALOS_API talos_status talos_linear_bwd(talos_ctx* ctx, const float* x, const fl
     auto hits = [&](const float* p, int64_t m) { return out && p && p < out + n && out < p + m; };
     return hits(dy, rows * out_f) || hits(act ? saved : nullptr, rows * out_f) || hits(x, rows * in_f) || hits(W, in_f * out_f);
   };
-  if (rows <= 4096 && rows * in_f * out_f <= (1LL << 26) && (dW || !db) && !(talos_switches() & SW_TC_NO_SMALL) && !over_input(dx, rows * in_f) &&
-      !over_input(dW, in_f * out_f) && !over_input(db, out_f) &&
-      talos_linear_bwd_small_launch(ctx, x, W, saved, dy, dx, dW, db, rows, in_f, out_f, act, accumulate))
-    return TALOS_OK;
+  const bool small = rows <= 4096 && rows * in_f * out_f <= (1LL << 26) && !(talos_switches() & SW_TC_NO_SMALL) && !over_input(dx, rows * in_f) &&
+                     !over_input(dW, in_f * out_f) && !over_input(db, out_f);
+  if (small && (dW || !db) && talos_linear_bwd_small_launch(ctx, x, W, saved, dy, dx, dW, db, rows, in_f, out_f, act, accumulate)) return TALOS_OK;
+  // (Up to that size the products stay on the CUDA cores in 3xTF32 mode at 2^26 itself, too: 64 x 2 048 x 512 40 -> 29 us.)
+  auto product_mode = [&](int64_t M, int64_t N, int64_t K) {
+    return small && mode == TALOS_MODE_TF32X3 && talos_gemm_small_walk(ctx, M, N, K) <= 1024 ? (int32_t)TALOS_MODE_FP32 : mode;
+  };
   const float* dz = dy;
   bool db_done = false;
   if (act != TALOS_ACT_NONE) {
@@ -90,11 +93,11 @@ TALOS_API talos_status talos_linear_bwd(talos_ctx* ctx, const float* x, const fl
   }
   if (dx) {   // dL/dx (+)= dZ . W^T   (src/autograd.rs:275-308)
     EpiArgs e{nullptr, nullptr, 0, nullptr, 0, 0, 0, accumulate & 1};
-    gemm_any(ctx, TALOS_OP_N, TALOS_OP_T, rows, in_f, out_f, dz, out_f, W, out_f, dx, in_f, mode, e);
+    gemm_any(ctx, TALOS_OP_N, TALOS_OP_T, rows, in_f, out_f, dz, out_f, W, out_f, dx, in_f, product_mode(rows, in_f, out_f), e);
   }
   if (dW) {   // dL/dW (+)= x^T . dZ   (src/autograd.rs:310-350)
     EpiArgs e{nullptr, nullptr, 0, nullptr, 0, 0, 0, (accumulate >> 1) & 1};
-    gemm_any(ctx, TALOS_OP_T, TALOS_OP_N, in_f, out_f, rows, x, in_f, dz, out_f, dW, out_f, mode, e);
+    gemm_any(ctx, TALOS_OP_T, TALOS_OP_N, in_f, out_f, rows, x, in_f, dz, out_f, dW, out_f, product_mode(in_f, out_f, rows), e);
   }
   if (db && !db_done) {   // dL/db (+)= column sums of dZ   (src/autograd.rs:539-543)
     talos_status st = talos_colsum(ctx, dz, db, rows, out_f, (accumulate >> 2) & 1);

@@ -228,14 +228,18 @@ talos_status talos_softmax_bwd(talos_ctx* ctx, const float* y, const float* dy, 
 /* ---- attention core: scores -> scale -> softmax -> .V ---------------------------------------- */
 /* q,k [BH,S,dqk], v [BH,S,dv], out [BH,S,dv]; probs (nullable) [BH,S,S] is written when the tape
  * needs it.  Replaces batched_matmul_qt_k + scale_tensor + softmax + batched_matmul_probs_v
- * (src/transformer.rs:539-550).  mode FP32: one fused CUDA-core kernel, scores never leave the SM,
- * S <= 128.  mode TF32 / TF32X3: two batched tensor-core GEMMs around an in-place softmax (S <= 1024);
- * shapes the tensor-core GEMM does not take fall back to the fused kernel. */
+ * (src/transformer.rs:539-550).  S <= 128, heads of 8 to 64, a multiple of 4, 16-byte aligned: one launch on the
+ * fp32 units with the scores on chip, in mode FP32 always, in the others where it is the faster route (few heads, S no
+ * multiple of 4, S <= 64).  Otherwise mode FP32: one fused CUDA-core kernel, S <= 128; mode TF32: one fused
+ * tensor-core kernel where its tiles fit, else, and in TF32X3, two batched tensor-core GEMMs around an in-place
+ * softmax (S <= 1024); shapes these do not take fall back to the fused CUDA-core kernel.  out may be q or k where
+ * it has their width. */
 talos_status talos_attention_fwd(talos_ctx* ctx, const float* q, const float* k, const float* v, float* out,
                                  float* probs, int64_t BH, int64_t S, int64_t dqk, int64_t dv, float scale,
                                  int32_t causal, int32_t mode);
 /* Backward from saved probs (the closures at src/transformer.rs:920-955, :1010-1046, :1063-1068,
- * :1098-1117): dq,dk,dv are overwritten.  The four products run as batched GEMMs in `mode`. */
+ * :1098-1117): dq,dk,dv are overwritten.  One launch on the fp32 units by the forward's rule, else four batched
+ * GEMMs in `mode`. */
 talos_status talos_attention_bwd(talos_ctx* ctx, const float* q, const float* k, const float* v,
                                  const float* probs, const float* dout, float* dq, float* dk, float* dv,
                                  int64_t BH, int64_t S, int64_t dqk, int64_t dvdim, float scale, int32_t mode);

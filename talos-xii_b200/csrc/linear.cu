@@ -8,8 +8,9 @@ __global__ void dact_mul_kernel(const float* __restrict__ dy, const float* __res
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dz[i] = dy[i] * talos_dact(saved[i], act);
 }
-// n a multiple of four, 16-byte aligned: two float4 a thread.  SiLU on [65536, 1024] 222 -> 114 us (its three 268 MB
-// streams take 123 us at the measured copy rate); one float a thread kept too few bytes in flight.
+// n a multiple of four, 16-byte aligned: two float4 a thread.  SiLU on [65536, 1024] 222 -> 114 us behind the product
+// that wrote dY (its three 268 MB streams take 123 us at the measured copy rate; the end of dY is still in L2); one float a
+// thread kept too few bytes in flight.
 template <int ACT>
 __global__ void __launch_bounds__(256)
 dact_mul_vec_kernel(const float4* __restrict__ dy, const float4* __restrict__ saved, float4* __restrict__ dz, long long n4) {

@@ -12,17 +12,16 @@ from gpu_util import TOL, dev, host, normal, rel_err
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("S,dqk,dv", [(1, 8, 8), (31, 16, 16), (32, 8, 20), (33, 32, 32), (50, 16, 16), (64, 32, 32), (65, 36, 12), (100, 48, 64), (127, 64, 64), (128, 16, 8),
-                                      (40, 68, 16), (40, 6, 7), (17, 4, 4)])
+SHAPES = [(1, 8, 8), (31, 16, 16), (32, 8, 20), (33, 32, 32), (50, 16, 16), (64, 32, 32), (65, 36, 12), (100, 48, 64), (127, 64, 64), (128, 16, 8), (40, 68, 16), (40, 6, 7),
+          (17, 4, 4)]
+
+
+# few heads; unaligned ones; more heads than SMs, on either side of the dispatch
+@pytest.mark.parametrize("S,dqk,dv,BH,offset", [s + (5, 0) for s in SHAPES] + [(50, 16, 16, 5, 1)] + [s + (300, 0) for s in SHAPES if s[0] in (64, 65, 100)])
 @pytest.mark.parametrize("causal", [0, 1])
 @pytest.mark.parametrize("mode", [0, 1, 2])
-@pytest.mark.parametrize("BH,offset", [(5, 0), (5, 1), (300, 0)])
-def test_forward_and_backward(talos, S, dqk, dv, causal, mode, BH, offset):
+def test_forward_and_backward(talos, S, dqk, dv, BH, offset, causal, mode):
     import torch
-    if offset and S != 50:
-        pytest.skip("unaligned heads: one shape is enough")
-    if BH > 5 and S not in (64, 65, 100):
-        pytest.skip("more heads than SMs: shapes on either side of the dispatch are enough")
     ctx, scale = talos.torch_context(0), 0.3
     q, k, v, do = normal(1, (BH, S, dqk)), normal(2, (BH, S, dqk)), normal(3, (BH, S, dv)), normal(4, (BH, S, dv))
     s = (q @ k.transpose(0, 2, 1)) * scale
@@ -61,13 +60,11 @@ def test_forward_and_backward(talos, S, dqk, dv, causal, mode, BH, offset):
     assert rel_err(host(bare[0])[offset:offset + ref["out"].size], ref["out"].ravel()) <= TOL[mode]
 
 
-@pytest.mark.parametrize("mode", [0, 1])
-@pytest.mark.parametrize("dqk,dv,result,source", [(16, 16, "out", "q"), (16, 16, "out", "v"), (16, 16, "dk", "q"), (16, 16, "dv", "do"), (32, 16, "out", "q"), (16, 32, "dk", "v")])
+@pytest.mark.parametrize("mode,dqk,dv,result,source", [(m, 16, 16) + rs for m in (0, 1) for rs in (("out", "q"), ("out", "v"), ("dk", "q"), ("dv", "do"))] +
+                         [(1, 32, 16, "out", "q"), (0, 16, 32, "dk", "v"), (1, 16, 32, "dk", "v")])
 def test_results_over_inputs(talos, mode, dqk, dv, result, source):
     # Head by head in place: the one-launch kernels.  At another width heads meet each other's: the separate products, whose order
     # allows it (fp32 mode has no such forward: its fused kernel, too, is one CTA a head).
-    if mode == 0 and dqk != dv and result == "out":
-        pytest.skip("heads of other widths over each other: tensor-core modes only")
     BH, S, scale = 300, 48, 0.3
     ctx, P, L = talos.torch_context(0), talos.ptr, talos.lib
     a = dict(q=normal(1, (BH, S, dqk)), k=normal(2, (BH, S, dqk)), v=normal(3, (BH, S, dv)), do=normal(4, (BH, S, dv)))

@@ -66,12 +66,16 @@ def test_binary_lengths(talos, ctx, n, offset, op):
 
 @pytest.mark.parametrize("act", ["relu", "tanh", "silu"])
 @pytest.mark.parametrize("rows,width", [(1, 4), (5, 3), (129, 16), (64, 65)])
-def test_linear_backward_without_bias_gradient(talos, ctx, act, rows, width):
-    # dZ = dY * act'(saved) as a pass of its own (no bias gradient asked for), seen through an identity weight: dX = dZ
+def test_linear_backward_without_bias_gradient(talos, ctx, act, rows, width, monkeypatch):
+    # dZ = dY * act'(saved) as a pass of its own (no bias gradient asked for, and not the one launch that takes layers of this
+    # size otherwise), in vectors and, for 15 elements, one by one; seen through an identity weight: dX = dZ
+    monkeypatch.setenv("TALOS_TC_NO_SMALL", "1")
     saved, dy = normal(8, (rows, width)) * 0.7, normal(9, (rows, width))
     eye = np.eye(width)
     bs, ps = _at(saved, 0); bd, pd = _at(dy, 0); be, pe = _at(eye, 0); bx, px = _at(np.zeros(rows * width), 0)
+    ctx.timeline_begin()
     talos.lib.talos_linear_bwd(ctx.handle, None, pe, ps, pd, px, None, None, rows, width, width, talos.ACTS[act], 0, 0)
+    assert [name for name, _ in ctx.timeline_end()][0] == "dact_mul"
     if act == "relu":
         d = (saved > 0).astype(np.float64)
     elif act == "tanh":

@@ -49,6 +49,23 @@ def gemm(talos, ctx, opA, opB, A, B, mode, C0=None, epi=None, ldpad=0):
     return c[:, :N]
 
 
+@pytest.fixture(params=["small", "tensor"])
+def route(request, monkeypatch):
+    """Products below 2^26 multiply-adds run on the CUDA cores in every mode; "tensor" takes that rule out, so that the
+    tensor-core kernels see the small sizes, too."""
+    if request.param == "tensor":
+        monkeypatch.setenv("TALOS_TC_NO_SMALL", "1")
+    return request.param
+
+
+def kernels(ctx, call):
+    """The result of `call` and the names of the launches it made (a context's first product runs the start-up check's, too)."""
+    call()
+    ctx.timeline_begin()
+    got = call()
+    return got, {name for name, _ in ctx.timeline_end()}
+
+
 def ref_gemm(opA, opB, A, B):
     return (A.T if opA else A) @ (B.T if opB else B)
 
@@ -69,7 +86,7 @@ def test_config1_gemm_512_all_forms(talos, ctx, mode):
 
 
 @pytest.mark.parametrize("mode", [0, 1, 2])
-def test_gemm_odd_shapes_all_ops(talos, ctx, mode):
+def test_gemm_odd_shapes_all_ops(talos, ctx, mode, route):
     sizes = [1, 3, 17, 63, 65, 127, 129]
     k = 0
     for M in sizes:
@@ -84,12 +101,14 @@ def test_gemm_odd_shapes_all_ops(talos, ctx, mode):
 
 
 @pytest.mark.parametrize("mode", [0, 1, 2])
-def test_gemm_aligned_rect_shapes(talos, ctx, mode):
+def test_gemm_aligned_rect_shapes(talos, ctx, mode, route):
     for (M, N, K) in [(256, 128, 64), (384, 256, 96), (1024, 16, 256), (128, 512, 1024), (4096, 256, 64), (640, 320, 200), (600, 512, 1056), (256, 1152, 1024)]:  # the last one has a B operand too large for the pre-split / pre-round path
         for opA, opB in [(0, 0), (0, 1), (1, 0), (1, 1)]:
             A = normal(M + K, (K, M) if opA else (M, K)); B = normal(N + K + 1, (N, K) if opB else (K, N))
-            got = gemm(talos, ctx, opA, opB, A, B, mode)
+            got, ran = kernels(ctx, lambda: gemm(talos, ctx, opA, opB, A, B, mode))
             assert rel_err(got, ref_gemm(opA, opB, A, B)) <= TOL[mode], (M, N, K, opA, opB)
+            tensor = mode != 0 and (route == "tensor" or M * N * K >= 2 ** 26)
+            assert ("gemm_tcgen05" in ran or "gemm_tcgen05_2cta" in ran) == tensor and ("gemm_small" in ran or mode == 0) != tensor, (M, N, K, ran)
 
 
 @pytest.mark.parametrize("mode", [0, 1, 2])
@@ -106,21 +125,23 @@ def test_gemm_split_k_dw_shape_and_determinism(talos, ctx, mode):
 
 
 @pytest.mark.parametrize("mode", [0, 1, 2])
-def test_gemm_epilogue_bias_act_aux(talos, ctx, mode):
+def test_gemm_epilogue_bias_act_aux(talos, ctx, mode, route):
     import torch
     M, N, K = 300, 256, 64
     A = normal(1, (M, K)); B = xavier(2, K, N); bias = normal(3, (N,), 0.1)
     for act in ("relu", "tanh", "silu"):
         z = torch.empty(M, N, device="cuda:0"); b = dev(bias)
         epi = talos.Epilogue(bias=talos.ptr(b), aux_out=talos.ptr(z), ld_aux_out=N, act=talos.ACTS[act])
-        y = gemm(talos, ctx, 0, 0, A, B, mode, epi=epi)
+        y, ran = kernels(ctx, lambda: gemm(talos, ctx, 0, 0, A, B, mode, epi=epi))
+        assert ("gemm_tcgen05" in ran) == (mode != 0 and route == "tensor"), ran
         zr = orc.bias_add(orc.matmul(A, B), bias)
         assert rel_err(z, zr) <= TOL[mode] and rel_err(y, om.act_fwd(zr, act)) <= TOL[mode], act
         # derivative epilogue: C = (A.B) * act'(saved)
         saved = zr if act == "silu" else om.act_fwd(zr, act)
         s = dev(saved)
         epi2 = talos.Epilogue(aux_in=talos.ptr(s), ld_aux_in=N, dact=talos.ACTS[act])
-        got = gemm(talos, ctx, 0, 0, A, B, mode, epi=epi2)
+        got, ran = kernels(ctx, lambda: gemm(talos, ctx, 0, 0, A, B, mode, epi=epi2))
+        assert ("gemm_tcgen05" in ran) == (mode != 0 and route == "tensor"), ran
         ref = om.act_bwd(orc.matmul(A, B), orc.f32r(zr), orc.f32r(om.act_fwd(zr, act)), act)
         assert rel_err(got, ref) <= max(TOL[mode], 2e-5), act
 

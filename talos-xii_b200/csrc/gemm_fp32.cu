@@ -196,8 +196,8 @@ void talos_gemm_fp32_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t
     splits = (int)std::min<int64_t>(ceil_div(2 * ctx->sm_count, tiles), K / 512);
     if (splits < 2) splits = 1;
   }
-  const bool in_place = talos_result_over_operand(opA, opB, M, N, K, A, lda, strideA, B, ldb, strideB, C, ldc, strideC, batch, epi);
-  if (!(M >= 96 && N >= 96) || (!in_place && (K < 256 || (tiles * 2 < ctx->sm_count && splits == 1)))) {
+  if (!(M >= 96 && N >= 96) || ((K < 256 || (tiles * 2 < ctx->sm_count && splits == 1)) &&
+                                !talos_result_over_operand(opA, opB, M, N, K, A, lda, strideA, B, ldb, strideB, C, ldc, strideC, batch, epi))) {
     talos_gemm_small_launch(ctx, opA, opB, M, N, K, A, lda, strideA, B, ldb, strideB, C, ldc, strideC, batch, epi);
     return;
   }

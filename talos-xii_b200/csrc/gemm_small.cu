@@ -358,7 +358,7 @@ void talos_gemm_small_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_
 #define TALOS_SMALL(BM, BN, TM, KG, KC) { if (vec) launch_gemm<BM, BN, TM, KG, KC, true>(ctx, g, batch); else launch_gemm<BM, BN, TM, KG, KC, false>(ctx, g, batch); }
   // Few tiles and a long reduction (a first layer's weight gradient over a large fp32 minibatch): a cluster's eight CTAs would
   // walk it alone, so it is cut into slabs, a cluster each, as many as fill the SMs; their results go through memory.
-  if (batch == 1 && talos_gemm_small_walk(ctx, M, N, K) > SLAB_WALK) {
+  if (batch == 1 && K > SLAB_WALK && talos_gemm_small_walk(ctx, M, N, K) > SLAB_WALK) {
     const SlabTile t = slab_tile(M, N);
     // as many clusters as there are slots, or fewer where the SMs then share them more evenly
     const int64_t tiles = small_tiles(M, N, t.bm, t.bn), sms = ctx->sm_count, most = t.ctas * sms / (8 * tiles);

@@ -515,7 +515,7 @@ void tc_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N, int64_t K
   // products of 8 192 x 256 x 256 otherwise leave 84 of 148 SMs idle while 64 run twice the columns (three-layer network
   // 64-256-256-16 on 8 192 rows, forward and backward: 180 -> 169 us).  The fused tanh' epilogue is built for 256 columns.
   if (!batched && !short_k && K < 16 * BK && !(extra && extra->tanh_saved) && !g_check_width && !(sw & SW_TC_FORCE_PAIR) &&
-      !talos_result_over_operand(opA, opB, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, epi))
+      !talos_result_over_operand(opA, opB, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, epi))      // (in place, one tile spans the columns)
     while (bn > 64 && ceil_div(M, BM) * ceil_div(N, bn / 2) <= ctx->sm_count) bn /= 2;
   TcArgs g;
   g.M = (int)M; g.N = (int)N; g.K = (int)K; g.C = C; g.ldc = ldc; g.epi = epi; g.status = ctx->dev_status; g.partial = nullptr;
@@ -797,9 +797,10 @@ bool talos_gemm_tc_launch(talos_ctx* ctx, int opA, int opB, int64_t M, int64_t N
   // reduction that a CTA would walk there is long: 30 x 1 448 x 1 448 22 us there, 20 here in 3xTF32 and 15 in TF32, 1 x 4 096 x
   // 4 096 48 against 31 and 19; at 1 024 that route is ahead (1 x 2 048 x 2 048 15 against 20).
   if ((((uintptr_t)A | (uintptr_t)B) & 15) || (lda & 3) || (ldb & 3) || K < 1) return false;
-  const bool small_ok = !extra && K <= 4096 && !(talos_switches() & SW_TC_NO_SMALL) && talos_gemm_small_walk(ctx, M, N, K) <= 1024 &&
-                        !talos_result_over_operand(opA, opB, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, epi);
-  if (M * N * K < (small_ok ? 1LL << 26 : 1LL << 18) || M < 1 || N < 1) return false;
+  if (M * N * K < (1LL << 18) || M < 1 || N < 1) return false;
+  if (M * N * K < (1LL << 26) && !extra && K <= 4096 && !(talos_switches() & SW_TC_NO_SMALL) && (K <= 1024 || talos_gemm_small_walk(ctx, M, N, K) <= 1024) &&
+      !talos_result_over_operand(opA, opB, M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, epi))
+    return false;
   if (!tc_ready(ctx)) return false;
   if (extra && extra->b_hi && ((((uintptr_t)extra->b_hi | (uintptr_t)extra->b_lo) & 15) != 0)) return false;
   tc_launch(ctx, opA, opB, M, N, K, A, lda, B, ldb, C, ldc, mode, epi, TcBatch{1, 0, 0, 0}, extra);

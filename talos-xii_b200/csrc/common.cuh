@@ -104,7 +104,7 @@ __device__ __forceinline__ void talos_pdl(T&... ptrs) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   ((void)([&] { asm volatile("" : "+l"(ptrs) : : "memory"); }()), ...);
 }
-// Launches `kern` (which must start with talos_pdl()) on the ctx stream, `cluster` CTAs to a cluster.  Follow it with talos_launched.
+// Launches `kern` (which must call talos_pdl() as said above) on the ctx stream, `cluster` CTAs to a cluster.  Follow it with talos_launched.
 template <typename... P, typename... A>
 inline void talos_kernel_cluster(talos_ctx* ctx, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, A&&... args) {
   cudaLaunchConfig_t cfg{};
